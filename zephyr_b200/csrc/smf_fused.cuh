@@ -105,8 +105,8 @@ template <typename R>
 __device__ __forceinline__ C4<R> hllc_fs(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
     const R cL = sqrt(eos.gamma * (L.p + eos.P0) * L.ri), cR = sqrt(eos.gamma * (Rs.p + eos.P0) * Rs.ri);
     // (the states are finite here: a NaN ordering of std::min does not arise)
-    const R SL = fmin(L.u - cL, Rs.u - cR);
-    const R SR = fmax(L.u + cL, Rs.u + cR);
+    const R SL = smin_t(L.u - cL, Rs.u - cR);
+    const R SR = smax_t(L.u + cL, Rs.u + cR);
     if (SL >= R(0)) return flux_x(L);
     if (SR <= R(0)) return flux_x(Rs);
     const R aL = L.r * (SL - L.u), aR = Rs.r * (SR - Rs.u);
@@ -136,8 +136,8 @@ __device__ __forceinline__ C4<R> hllc_fs(const FS<R> &L, const FS<R> &Rs, const 
 template <typename R>
 __device__ __forceinline__ C4<R> hll_fs(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
     const R cL = sqrt(eos.gamma * (L.p + eos.P0) * L.ri), cR = sqrt(eos.gamma * (Rs.p + eos.P0) * Rs.ri);
-    const R SL = fmin(L.u - cL, fmin(Rs.u - cR, R(0)));
-    const R SR = fmax(L.u + cL, fmax(Rs.u + cR, R(0)));
+    const R SL = smin_t(smin_t(L.u - cL, Rs.u - cR), R(0));
+    const R SR = smax_t(smax_t(L.u + cL, Rs.u + cR), R(0));
     const C4<R> FL = flux_x(L), FR = flux_x(Rs);
     const R EL = L.e + R(0.5) * (L.u * L.u + L.v * L.v);
     const R ER = Rs.e + R(0.5) * (Rs.u * Rs.u + Rs.v * Rs.v);
@@ -233,7 +233,7 @@ struct FusedLayout {
     static constexpr size_t off_wt = off_zin + zin_bytes;
     static constexpr size_t wt_bytes = al(GR * GC);
     static constexpr size_t off_red = off_wt + wt_bytes;
-    static constexpr size_t bytes = off_red + al(8 * GR);
+    static constexpr size_t bytes = off_red + al(16 + 4 * GR);  // dt / V, a CFL minimum, a bound per warp
 };
 
 // x wrapped into [0, n) for any x (the Z region reaches two cells beyond the
@@ -259,8 +259,38 @@ __device__ __forceinline__ bool z_cell(const StructMesh &m, int i0, int j0, int 
     return true;
 }
 
-template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
-__global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<R> f) {
+// Quotients that are the same for every cell, formed once on the host (an
+// FP64 division is some 25 instructions: the seven of them that each thread
+// used to form were a tenth of the kernel's instructions).
+template <typename R>
+struct StepConst {
+    R halfx, halfy;    // h / 2
+    R inv2hx, inv2hy;  // 1 / 2h
+    R invhx, invhy;    // 1 / h
+    R igm1;            // 1 / (gamma - 1)
+};
+template <typename R>
+inline StepConst<R> step_const(const SmfArgs &a) {
+    const StructMesh &m = a.mesh;
+    return StepConst<R>{R(0.5 * m.hx), R(0.5 * m.hy), R(0.5 / m.hx),      R(0.5 / m.hy),
+                        R(1.0 / m.hx), R(1.0 / m.hy), R(1.0 / a.eos.gm1)};
+}
+
+// A lower bound of the CFL term dinc / (|v| + c) in FP32: dinc^2 and the
+// squares of the two speeds rounded to FP32, each step within a few 2^-24,
+// the quotient taken 2e-4 too small.  0 where FP32 cannot hold the squares
+// (the caller then takes the FP64 term).
+__device__ __forceinline__ float cfl_lower(double dinc2, double c2, double v2) {
+    const float d = sqrtf((float)dinc2), s = sqrtf((float)c2) + sqrtf((float)v2);
+    const bool in_range = d > 1e-15f && d < 1e15f && s > 1e-10f && s < 1e15f;
+    return in_range ? __fdividef(d, s) * 0.9998f : 0.0f;
+}
+
+// One block's tile.  INTERIOR: the whole Z region lies inside the mesh (no
+// boundary face, no wrapped index), so the boundary selects, the wrapping and
+// the domain marks drop out.
+template <typename R, bool MIXED, int MODE, int LIM, int TH, bool INTERIOR>
+__device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, const StepConst<R> &k) {
     using L = FusedLayout<R, TH, MODE>;
     constexpr int ZR = L::ZR, ZC = L::ZC, GR = L::GR, GC = L::GC, NT = L::NT;
     constexpr bool PC = MODE == FUSED_PC;
@@ -279,10 +309,7 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
     const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l;
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
     const EosR<R> eos = eos_as<R>(a.eos);
-    const R igm1 = R(1.0 / a.eos.gm1);
-    // per-axis geometry of the uniform rectangle
-    const R halfx = R(0.5 * m.hx), halfy = R(0.5 * m.hy);
-    const R inv2hx = R(0.5 / m.hx), inv2hy = R(0.5 / m.hy), invhx = R(1.0 / m.hx), invhy = R(1.0 / m.hy);
+    const R igm1 = k.igm1, halfx = k.halfx, halfy = k.halfy;
     // source of the stage: the state at t^n, or the Heun stage value z*
     const R *const *src = MODE == FUSED_HEUN_B ? const_cast<const R *const *>(f.h) : f.w;
 
@@ -293,24 +320,46 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
     const double dt = step_dt(a, f.slot_cur);
 
     // ---- phase 0: stage Z ----------------------------------------------------
-    for (int k = tid; k < ZR * ZC; k += NT) {
-        const int zr = k / ZC, zc = k - zr * ZC;
-        int gi, gj;
-        const bool in = z_cell(m, i0, j0, zr, zc, gi, gj);
-        zin[zr][zc] = in;
-        if (in) {
-            const int g = gi * m.ny + gj;
+    if (INTERIOR) {
+        // row by row: 32 columns by every warp, the last two by its low lanes
+        const R *p0 = src[0], *p1 = src[1], *p2 = src[2], *p3 = src[3], *p4 = src[4];
+        for (int zr = r; zr < ZR; zr += GR) {
+            int g = (i0 + zr - 2) * m.ny + j0 - 2 + l;
 #pragma unroll
-            for (int q = 0; q < 5; ++q) Z[q][zr][zc] = src[q][g];
+            for (int zc = l; zc < ZC; zc += 32, g += 32) {
+                Z[0][zr][zc] = p0[g];
+                Z[1][zr][zc] = p1[g];
+                Z[2][zr][zc] = p2[g];
+                Z[3][zr][zc] = p3[g];
+                Z[4][zr][zc] = p4[g];
+            }
+        }
+    } else {
+        for (int k = tid; k < ZR * ZC; k += NT) {
+            const int zr = k / ZC, zc = k - zr * ZC;
+            int gi, gj;
+            const bool in = z_cell(m, i0, j0, zr, zc, gi, gj);
+            zin[zr][zc] = in;
+            if (in) {
+                const int g = gi * m.ny + gj;
+#pragma unroll
+                for (int q = 0; q < 5; ++q) Z[q][zr][zc] = src[q][g];
+            }
         }
     }
+    // dt / V once per block, and the next step's CFL minimum so far
+    if (tid == 0) {
+        red[0] = dbits(dt / m.vol);
+        if (MODE != FUSED_HEUN_A) red[1] = __ldcg(f.slot_nxt);
+    }
     __syncthreads();
+    const double coef = __longlong_as_double((long long)red[0]);
 
     // ---- phase 1: gradients (and the half step) of the G cell (r, l) ---------
-    if (zin[r + 1][l + 1]) {
+    if (INTERIOR || zin[r + 1][l + 1]) {
         int gi = i0 - 1 + r, gj = j0 - 1 + l;  // wrapped global coordinates
-        if (m.xper) gi = wrap_idx(gi, m.nx);
-        if (m.yper) gj = wrap_idx(gj, m.ny);
+        if (!INTERIOR && m.xper) gi = wrap_idx(gi, m.nx);
+        if (!INTERIOR && m.yper) gj = wrap_idx(gj, m.ny);
         const int zr = r + 1, zc = l + 1;
         // conserved state of the cell at t^n (predictor-corrector): FAST from
         // the staged primitive state, MIXED from the FP64 fields (loaded here,
@@ -326,10 +375,10 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
             }
         }
         // boundary flags of the four slots (the normals are the axes)
-        const int fL = gi > 0 ? BC_INNER : m.bc[0];
-        const int fR = gi < m.nx - 1 ? BC_INNER : m.bc[1];
-        const int fB = gj > 0 ? BC_INNER : m.bc[2];
-        const int fT = gj < m.ny - 1 ? BC_INNER : m.bc[3];
+        const int fL = INTERIOR || gi > 0 ? BC_INNER : m.bc[0];
+        const int fR = INTERIOR || gi < m.nx - 1 ? BC_INNER : m.bc[1];
+        const int fB = INTERIOR || gj > 0 ? BC_INNER : m.bc[2];
+        const int fT = INTERIOR || gj < m.ny - 1 ? BC_INNER : m.bc[3];
         const bool bL = is_boundary(fL), bR = is_boundary(fR), bB = is_boundary(fB), bT = is_boundary(fT);
         R gx[4], gy[4];
 #pragma unroll
@@ -341,8 +390,8 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
             const R nR = bR ? ((q == 1 && fR == BC_WALL) ? -c : c) : Z[q][zr + 1][zc];
             const R nB = bB ? ((q == 2 && fB == BC_WALL) ? -c : c) : Z[q][zr][zc - 1];
             const R nT = bT ? ((q == 2 && fT == BC_WALL) ? -c : c) : Z[q][zr][zc + 1];
-            gx[q] = slope<LIM, R>(a.limiter, nL - c, nR - c, inv2hx, invhx);
-            gy[q] = slope<LIM, R>(a.limiter, nB - c, nT - c, inv2hy, invhy);
+            gx[q] = slope<LIM, R>(a.limiter, nL - c, nR - c, k.inv2hx, k.invhx);
+            gy[q] = slope<LIM, R>(a.limiter, nB - c, nT - c, k.inv2hy, k.invhy);
             G[q][r][l] = gx[q];
             G[4 + q][r][l] = gy[q];
         }
@@ -381,12 +430,12 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
                     F[2] += (double)lf.mv * w;
                     F[3] += (double)lf.E * w;
                 }
-                const double coef = 0.5 * dt / m.vol;
+                const double half = 0.5 * coef;
                 C4<double> q = q0;
-                q.r -= coef * F[0];
-                q.mu -= coef * F[1];
-                q.mv -= coef * F[2];
-                q.E -= coef * F[3];
+                q.r -= half * F[0];
+                q.mu -= half * F[1];
+                q.mv -= half * F[2];
+                q.E -= half * F[3];
                 double ri;
                 const P5<double> hd = prim_ri(q, a.eos, ri);
                 if (!bad64(hd, a.eos)) hz = down<R>(hd);
@@ -475,20 +524,20 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
     // (predictor-corrector: the fluxes overwrite Z, which no thread reads
     // after phase 1)
     if (r <= TH && l >= 1 && l <= 30) {  // +x face between G cells (r, l) and (r + 1, l)
-        const bool inA = zin[r + 1][l + 1], inB = zin[r + 2][l + 1];
+        const bool inA = INTERIOR || zin[r + 1][l + 1], inB = INTERIOR || zin[r + 2][l + 1];
         C4<R> lf{R(0), R(0), R(0), R(0)};
         if (inA && inB) lf = face_interior(std::integral_constant<int, 0>{});
-        else if (inA || inB) lf = face_boundary(0, inA);
+        else if (!INTERIOR && (inA || inB)) lf = face_boundary(0, inA);
         FX[0][r][l] = lf.r;
         FX[1][r][l] = lf.mu;
         FX[2][r][l] = lf.mv;
         FX[3][r][l] = lf.E;
     }
     if (r >= 1 && r <= TH && l <= 30) {  // +y face between G cells (r, l) and (r, l + 1)
-        const bool inA = zin[r + 1][l + 1], inB = zin[r + 1][l + 2];
+        const bool inA = INTERIOR || zin[r + 1][l + 1], inB = INTERIOR || zin[r + 1][l + 2];
         C4<R> lf{R(0), R(0), R(0), R(0)};
         if (inA && inB) lf = face_interior(std::integral_constant<int, 1>{});
-        else if (inA || inB) lf = face_boundary(1, inA);
+        else if (!INTERIOR && (inA || inB)) lf = face_boundary(1, inA);
         FY[0][r - 1][l] = lf.r;
         FY[1][r - 1][l] = lf.mu;
         FY[2][r - 1][l] = lf.mv;
@@ -497,16 +546,16 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
     __syncthreads();
 
     // ---- phase 3: update of the interior cells --------------------------------
-    unsigned long long best = 0x7FEFFFFFFFFFFFFFull;
+    float low = INFINITY;  // lower bound of the cell's CFL term (0: none; infinite: no cell)
+    P5<double> zn{};
     const int i = i0 - 1 + r, j = j0 - 1 + l;
-    if (r >= 1 && r <= TH && l >= 1 && l <= 30 && i < m.nx && j < m.ny) {
+    if (r >= 1 && r <= TH && l >= 1 && l <= 30 && (INTERIOR || (i < m.nx && j < m.ny))) {
         const int ic = i * m.ny + j;
         const double hy = m.hy, hx = m.hx;
         double F[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             F[k] = ((-FX[k][r - 1][l] * hy + FX[k][r][l] * hy) - FY[k][r - 1][l - 1] * hx) + FY[k][r - 1][l] * hx;
-        const double coef = dt / m.vol;
         C4<double> q;
         if (PC) {
             q = C4<double>{Q[0][r][l], Q[1][r][l], Q[2][r][l], Q[3][r][l]};
@@ -530,7 +579,7 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
             q.E = 0.5 * (q0.E + q.E);
         }
         double ri;
-        P5<double> zn = prim_ri(q, a.eos, ri);
+        zn = prim_ri(q, a.eos, ri);
         if (MODE == FUSED_HEUN_A) {
             st5(f.h, ic, down<R>(zn));  // Heun stage value
         } else {
@@ -555,24 +604,36 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
                 f.qn[3][ic] = q.E;
             }
             st5(f.wn, ic, down<R>(zn));
-            // CFL term of the new state for the next step (sm_fluid.cpp:104-111),
-            // with the arithmetic of k_cfl, which takes the minimum after an
-            // upload or a halo exchange: the same state gives the same dt
-            const double c = sqrt(a.eos.gamma * (zn.p + a.eos.P0) / zn.r);
-            const double dinc = sqrt(smin(m.inc2x[i], m.inc2y[j]));
-            const double lam = dinc / (sqrt(zn.u * zn.u + zn.v * zn.v) + c);
-            if (lam >= 0.0) best = dbits(lam);
+            low = cfl_lower(smin(m.inc2x[i], m.inc2y[j]), a.eos.gamma * (zn.p + a.eos.P0) * ri,
+                            zn.u * zn.u + zn.v * zn.v);
         }
     }
+    // The minimum of the CFL terms of the new state for the next step
+    // (sm_fluid.cpp:104-111), with the arithmetic of k_cfl, which takes the
+    // minimum after an upload or a halo exchange: the same state gives the
+    // same dt.  That term (two divisions and three square roots in FP64) is
+    // formed only where its FP32 lower bound does not exceed the block's
+    // smallest and the minimum that other blocks have reached: a larger
+    // bound cannot hold the minimum.
     if (MODE != FUSED_HEUN_A) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long t2 = __shfl_xor_sync(0xffffffffu, best, o);
-            best = t2 < best ? t2 : best;
-        }
-        if (l == 0) red[r] = best;
+        float wmin = low > 0.0f ? low : INFINITY;
+        for (int o = 16; o > 0; o >>= 1) wmin = fminf(wmin, __shfl_xor_sync(0xffffffffu, wmin, o));
+        float *redf = reinterpret_cast<float *>(red + 2);
+        if (l == 0) redf[r] = wmin;
         __syncthreads();
-        if (r == 0) {
-            best = l < GR ? red[l] : 0x7FEFFFFFFFFFFFFFull;
+        float lim = redf[l < GR ? l : 0];
+        for (int o = 16; o > 0; o >>= 1) lim = fminf(lim, __shfl_xor_sync(0xffffffffu, lim, o));
+        // 1.0005: the bound is at most 3e-4 below its term
+        lim = fminf(lim * 1.0005f, __double2float_ru(__longlong_as_double((long long)red[1])));
+        const bool take = low <= lim && low < INFINITY;
+        if (__any_sync(0xffffffffu, take)) {
+            unsigned long long best = 0x7FEFFFFFFFFFFFFFull;
+            if (take) {
+                const double c = sqrt(a.eos.gamma * (zn.p + a.eos.P0) / zn.r);
+                const double dinc = sqrt(smin(m.inc2x[i], m.inc2y[j]));
+                const double lam = dinc / (sqrt(zn.u * zn.u + zn.v * zn.v) + c);
+                if (lam >= 0.0) best = dbits(lam);
+            }
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long t2 = __shfl_xor_sync(0xffffffffu, best, o);
                 best = t2 < best ? t2 : best;
@@ -580,6 +641,15 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
             if (l == 0) atomicMin(f.slot_nxt, best);
         }
     }
+}
+
+template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
+__global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<R> f, StepConst<R> k) {
+    const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
+    if (i0 >= 2 && i0 + TH + 2 <= a.mesh.nx && j0 >= 2 && j0 + 32 <= a.mesh.ny)
+        step_tile<R, MIXED, MODE, LIM, TH, true>(a, f, k);
+    else
+        step_tile<R, MIXED, MODE, LIM, TH, false>(a, f, k);
 }
 
 // Launch one stage of the fused step on `stream` (dynamic shared memory of
@@ -597,7 +667,7 @@ inline void launch_fused_stage(const SmfArgs &a, const Fields<R> &f, cudaStream_
     }
     dim3 block(32, TH + 2);
     dim3 grid((a.mesh.ny + 29) / 30, (a.mesh.nx + TH - 1) / TH);
-    kern<<<grid, block, L::bytes, s>>>(a, f);
+    kern<<<grid, block, L::bytes, s>>>(a, f, step_const<R>(a));
 }
 
 // One stage (FUSED_PC, FUSED_HEUN_A or FUSED_HEUN_B) with the limiter

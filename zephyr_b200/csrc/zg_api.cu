@@ -1040,6 +1040,7 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
     m.fym = c->d_geo + ofy;
     m.inc2x = c->d_geo + oix;
     m.inc2y = c->d_geo + oiy;
+    m.inc2min = std::min(*std::min_element(i2x.begin(), i2x.end()), *std::min_element(i2y.begin(), i2y.end()));
     c->box[0] = x_min;
     c->box[1] = x_max;
     c->box[2] = y_min;
