@@ -43,6 +43,7 @@ UNITS = {
     # scalar VOF transport: polygon clipping and sections bit-exact with the reference
     "tr_vof.cu": ["-fmad=false"],
     "zg_vtu.cu": [],
+    "host_copy.cu": [],
     "smf_fast.cu": [],
     "smf_slot_fast.cu": [],
     "smf_slot_order.cu": [],

@@ -445,6 +445,33 @@ __global__ void __launch_bounds__(BLOCK) k_make_states(MmArgs a, const double *r
     store(a.z, ic, state_of_rvp(a.mix, rho[ic], vx[ic], vy[ic], P[ic], b));
 }
 
+// The state as 14 doubles per cell (zg_mmf_state_download's layout; absent
+// materials: fraction 0, true density NaN), two lanes a row of 16-byte stores.
+__global__ void __launch_bounds__(BLOCK) k_pack_states(MmField z, int n, double2 *cells) {
+    const long long t = (long long)blockIdx.x * BLOCK + threadIdx.x;
+    const int ic = (int)(t / 7), q = (int)(t - 7LL * ic);
+    if (ic >= n) return;
+    static_assert(NM == 2, "pairs of the two materials' entries");
+    double2 v = make_double2(0.0, 0.0);
+    if (q == 0) v = make_double2(z.rho[ic], z.vx[ic]);
+    else if (q == 1) v = make_double2(z.vy[ic], z.P[ic]);
+    else if (q == 2) v = make_double2(z.e[ic], z.T[ic]);
+    else if (q == 3) v = make_double2(z.b[0][ic], z.b[1][ic]);
+    else if (q == 5) v = make_double2(z.r[0][ic], z.r[1][ic]);
+    else if (q == 6) v = make_double2(CUDART_NAN, CUDART_NAN);
+    cells[t] = v;
+}
+__global__ void __launch_bounds__(BLOCK) k_pack_planes(MmArgs a, double *normals, double *offsets) {
+    const int ic = blockIdx.x * BLOCK + threadIdx.x;
+    if (ic >= a.mesh.n) return;
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+        normals[((size_t)ic * NM + i) * 2] = a.nrm_x[i][ic];
+        normals[((size_t)ic * NM + i) * 2 + 1] = a.nrm_y[i][ic];
+        offsets[(size_t)ic * NM + i] = a.off[i][ic];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Second order (MmFluid::integrate with accuracy 2, mm_fluid.cpp:152-168).
 // The state as an array of NG components; the reference's mmf::PState also
@@ -982,6 +1009,14 @@ void launch_flags(const MmArgs &a, int *flags, void *stream) {
 void launch_make_states(const MmArgs &a, const double *rho, const double *vx, const double *vy, const double *P,
                         const double *beta, void *stream) {
     k_make_states<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a, rho, vx, vy, P, beta);
+}
+void launch_pack_states(const MmField &z, int n, double *cells, void *stream) {
+    const long long t = 7LL * n;
+    k_pack_states<<<(unsigned)((t + BLOCK - 1) / BLOCK), BLOCK, 0, (cudaStream_t)stream>>>(
+        z, n, reinterpret_cast<double2 *>(cells));
+}
+void launch_pack_planes(const MmArgs &a, double *normals, double *offsets, void *stream) {
+    k_pack_planes<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a, normals, offsets);
 }
 
 }  // namespace mmf

@@ -86,6 +86,10 @@ void launch_stage1(const MmArgs &a, void *stream);
 void launch_stage2(const MmArgs &a, void *stream);
 void launch_make_states(const MmArgs &a, const double *rho, const double *vx, const double *vy, const double *P,
                         const double *beta, void *stream);
+// the n cell states as the 14 doubles per cell of zg_mmf_state_download, and
+// the interface planes as zg_mmf_interface's arrays
+void launch_pack_states(const MmField &z, int n, double *cells, void *stream);
+void launch_pack_planes(const MmArgs &a, double *normals, double *offsets, void *stream);
 
 }  // namespace mmf
 }  // namespace zg

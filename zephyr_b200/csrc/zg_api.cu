@@ -15,6 +15,7 @@
 
 #include "../../include/zephyr_gpu.h"
 #include "amr_refine.h"
+#include "host_copy.h"
 #include "mmf_types.h"
 #include "smf_tiled.cuh"
 #include "smf_tiled_launch.h"
@@ -912,6 +913,7 @@ int zg_create(zg_ctx **out, int device) {
         return ZG_ERR_CUDA;
     }
     c->stream = c->own_stream;
+    host::retain();
     *out = c;
     return ZG_OK;
 }
@@ -929,6 +931,7 @@ int zg_destroy(zg_ctx *c) {
         if (c->side) cudaStreamDestroy(c->side);
         for (cudaEvent_t e : {c->ev_fork, c->ev_join, c->ev_cleared, c->ev_dt})
             if (e) cudaEventDestroy(e);
+        host::release();
     }
     delete c;
     return ZG_OK;
@@ -1269,11 +1272,9 @@ int zg_state_download(zg_ctx *c, double *rho, double *vx, double *vy, double *p,
     int rc = materialize_prim(c);
     if (rc != ZG_OK) return rc;
     size_t bytes = (size_t)c->n * sizeof(double);
-    double *dst[5] = {rho, vx, vy, p, e};
-    const double *src[5] = {c->z.r, c->z.u, c->z.v, c->z.p, c->z.e};
-    for (int k = 0; k < 5; ++k)
-        ZG_CUDA(c, cudaMemcpyAsync(dst[k], src[k], bytes, cudaMemcpyDeviceToHost, c->stream));
-    ZG_CUDA(c, cudaStreamSynchronize(c->stream));
+    const host::Piece out[5] = {
+        {rho, c->z.r, bytes}, {vx, c->z.u, bytes}, {vy, c->z.v, bytes}, {p, c->z.p, bytes}, {e, c->z.e, bytes}};
+    ZG_CUDA(c, host::copy(c->device, c->stream, out, 5, true));
     return ZG_OK;
 }
 
@@ -1859,24 +1860,14 @@ int zg_mmf_state_download(zg_ctx *c, double *cells) {
     if (!cells) return fail(c, ZG_ERR_ARG, "zg_mmf_state_download: null array");
     DeviceGuard g(c->device);
     size_t n = (size_t)c->n;
-    std::vector<double *> fields = {c->mz.rho, c->mz.vx, c->mz.vy, c->mz.P, c->mz.e, c->mz.T};
-    for (int k = 0; k < mmf::NMAT; ++k) fields.push_back(c->mz.b[k]);
-    for (int k = 0; k < mmf::NMAT; ++k) fields.push_back(c->mz.r[k]);
-    std::vector<double> soa(fields.size() * n);
-    for (size_t k = 0; k < fields.size(); ++k)
-        ZG_CUDA(c, cudaMemcpyAsync(soa.data() + k * n, fields[k], n * sizeof(double), cudaMemcpyDeviceToHost,
-                                   c->stream));
-    rc = mm_check_error(c);
-    const double nan = std::numeric_limits<double>::quiet_NaN();
-    for (size_t i = 0; i < n; ++i) {
-        double *s = cells + 14 * i;
-        for (int k = 0; k < 6; ++k) s[k] = soa[k * n + i];
-        for (int k = 0; k < 4; ++k) {
-            s[6 + k] = k < mmf::NMAT ? soa[(6 + k) * n + i] : 0.0;
-            s[10 + k] = k < mmf::NMAT ? soa[(6 + mmf::NMAT + k) * n + i] : nan;
-        }
-    }
-    return rc;
+    // packed on the device, in the work space of the steps (60 doubles per
+    // cell; the stream's earlier steps are done with it)
+    mmf::launch_pack_states(c->mz, c->n, c->d_mm_qbuf, (void *)c->stream);
+    ++c->launches;
+    ZG_CUDA(c, cudaGetLastError());
+    const host::Piece out{cells, c->d_mm_qbuf, 14 * n * sizeof(double)};
+    ZG_CUDA(c, host::copy(c->device, c->stream, &out, 1, true));
+    return mm_check_error(c);
 }
 
 int zg_mmf_grad_a(zg_ctx *c, double *out) {
@@ -1906,21 +1897,20 @@ int zg_mmf_make_states(zg_ctx *c, const double *rho, const double *vx, const dou
     for (size_t i = 0; i < n; ++i)
         for (int k = mmf::NMAT; k < 4; ++k)
             if (beta[4 * i + k] != 0.0) return fail(c, ZG_ERR_ARG, "zg_mmf_make_states: fraction of an absent material");
-    // staging: rho, vx, vy, p (n each) and beta (4 n) in the next-state buffer's fields
-    double *tmp = nullptr;
-    ZG_CUDA(c, cudaMalloc(&tmp, 8 * n * sizeof(double)));
-    const double *src[4] = {rho, vx, vy, p};
-    for (int k = 0; k < 4; ++k)
-        ZG_CUDA(c, cudaMemcpyAsync(tmp + k * n, src[k], n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    ZG_CUDA(c, cudaMemcpyAsync(tmp + 4 * n, beta, 4 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    // staging: rho, vx, vy, p (n each) and beta (4 n) in the steps' work space
+    double *tmp = c->d_mm_qbuf;
+    const size_t bytes = n * sizeof(double);
+    const host::Piece in[5] = {{const_cast<double *>(rho), tmp, bytes},
+                               {const_cast<double *>(vx), tmp + n, bytes},
+                               {const_cast<double *>(vy), tmp + 2 * n, bytes},
+                               {const_cast<double *>(p), tmp + 3 * n, bytes},
+                               {const_cast<double *>(beta), tmp + 4 * n, 4 * bytes}};
+    ZG_CUDA(c, host::copy(c->device, c->stream, in, 5, false));
     mmf::MmArgs a = make_mm_args(c);
     mmf::launch_make_states(a, tmp, tmp + n, tmp + 2 * n, tmp + 3 * n, tmp + 4 * n, (void *)c->stream);
     ++c->launches;
-    cudaError_t e = cudaGetLastError();
-    cudaError_t s = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
-    if (e != cudaSuccess) return cuda_fail(c, e, "zg_mmf_make_states launch");
-    if (s != cudaSuccess) return cuda_fail(c, s, "zg_mmf_make_states");
+    ZG_CUDA(c, cudaGetLastError());
+    ZG_CUDA(c, cudaStreamSynchronize(c->stream));
     return ZG_OK;
 }
 
@@ -1971,22 +1961,13 @@ int zg_mmf_interface(zg_ctx *c, double *normals, double *offsets) {
     ++c->launches;
     ZG_CUDA(c, cudaGetLastError());
     size_t n = (size_t)c->n;
-    std::vector<double> buf(3 * mmf::NMAT * n);
-    for (int i = 0; i < mmf::NMAT; ++i) {
-        ZG_CUDA(c, cudaMemcpyAsync(buf.data() + (3 * i) * n, c->mnx[i], n * sizeof(double), cudaMemcpyDeviceToHost,
-                                   c->stream));
-        ZG_CUDA(c, cudaMemcpyAsync(buf.data() + (3 * i + 1) * n, c->mny[i], n * sizeof(double),
-                                   cudaMemcpyDeviceToHost, c->stream));
-        ZG_CUDA(c, cudaMemcpyAsync(buf.data() + (3 * i + 2) * n, c->moff[i], n * sizeof(double),
-                                   cudaMemcpyDeviceToHost, c->stream));
-    }
-    ZG_CUDA(c, cudaStreamSynchronize(c->stream));
-    for (size_t ic = 0; ic < n; ++ic)
-        for (int i = 0; i < mmf::NMAT; ++i) {
-            normals[(ic * mmf::NMAT + i) * 2] = buf[(3 * i) * n + ic];
-            normals[(ic * mmf::NMAT + i) * 2 + 1] = buf[(3 * i + 1) * n + ic];
-            offsets[ic * mmf::NMAT + i] = buf[(3 * i + 2) * n + ic];
-        }
+    double *nrm = c->d_mm_qbuf, *off = nrm + 2 * mmf::NMAT * n;  // the steps' work space
+    mmf::launch_pack_planes(a, nrm, off, (void *)c->stream);
+    ++c->launches;
+    ZG_CUDA(c, cudaGetLastError());
+    const host::Piece out[2] = {{normals, nrm, 2 * mmf::NMAT * n * sizeof(double)},
+                                {offsets, off, mmf::NMAT * n * sizeof(double)}};
+    ZG_CUDA(c, host::copy(c->device, c->stream, out, 2, true));
     return ZG_OK;
 }
 
@@ -2141,8 +2122,8 @@ int zg_tr_upload(zg_ctx *c, const double *u1) {
     if (rc != ZG_OK) return rc;
     if (!u1) return fail(c, ZG_ERR_ARG, "zg_tr_upload: null array");
     DeviceGuard g(c->device);
-    ZG_CUDA(c, cudaMemcpyAsync(c->targs.u, u1, (size_t)c->n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    ZG_CUDA(c, cudaStreamSynchronize(c->stream));
+    const host::Piece in{const_cast<double *>(u1), c->targs.u, (size_t)c->n * sizeof(double)};
+    ZG_CUDA(c, host::copy(c->device, c->stream, &in, 1, false));
     return ZG_OK;
 }
 
@@ -2152,20 +2133,24 @@ int zg_tr_download(zg_ctx *c, double *u1, double *nrm, double *pt) {
     DeviceGuard g(c->device);
     const size_t n = (size_t)c->n;
     const tr::TrArgs &a = c->targs;
-    std::vector<double> buf(4 * n);
-    if (u1) ZG_CUDA(c, cudaMemcpyAsync(u1, a.u, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    // the current buffers' nx, ny, px, py are contiguous
-    if (nrm || pt)
-        ZG_CUDA(c, cudaMemcpyAsync(buf.data(), a.nx[a.cur], 4 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    ZG_CUDA(c, cudaStreamSynchronize(c->stream));
-    for (size_t i = 0; i < n && (nrm || pt); ++i) {
-        if (nrm) {
-            nrm[2 * i] = buf[i];
-            nrm[2 * i + 1] = buf[n + i];
-        }
-        if (pt) {
-            pt[2 * i] = buf[2 * n + i];
-            pt[2 * i + 1] = buf[3 * n + i];
+    if (u1) {
+        const host::Piece out{u1, a.u, n * sizeof(double)};
+        ZG_CUDA(c, host::copy(c->device, c->stream, &out, 1, true));
+    }
+    if (nrm || pt) {
+        // the current buffers' nx, ny, px, py are contiguous
+        std::vector<double> buf(4 * n);
+        const host::Piece out{buf.data(), a.nx[a.cur], 4 * n * sizeof(double)};
+        ZG_CUDA(c, host::copy(c->device, c->stream, &out, 1, true));
+        for (size_t i = 0; i < n; ++i) {
+            if (nrm) {
+                nrm[2 * i] = buf[i];
+                nrm[2 * i + 1] = buf[n + i];
+            }
+            if (pt) {
+                pt[2 * i] = buf[2 * n + i];
+                pt[2 * i + 1] = buf[3 * n + i];
+            }
         }
     }
     return tr_check_error(c);
