@@ -105,6 +105,15 @@ struct MixD {
     MatD mat[NM];
 };
 
+// Volume fraction b rho / r of a material with mass fraction b and true density
+// r, within [0, 1]; 0 where r is NaN (an absent material).  The division never
+// sees the NaN or a zero numerator (div_z).
+__device__ __forceinline__ double volume_fraction(double b, double rho, double r) {
+    const bool absent = isnan(r);
+    const double q = div_z(b * rho, absent ? 1.0 : r);
+    return absent ? 0.0 : fmax_std(0.0, fmin_std(q, 1.0));
+}
+
 // ---------------------------------------------------------------------------
 // Fractions
 template <int NM>
@@ -133,7 +142,7 @@ __device__ __forceinline__ void cutoff(Frac<NM> &b, double eps) {
         sum += b.f[i];
     }
 #pragma unroll
-    for (int i = 0; i < NM; ++i) b.f[i] /= sum;
+    for (int i = 0; i < NM; ++i) b.f[i] = div_z(b.f[i], sum);
 }
 template <int NM>
 __device__ __forceinline__ void normalize(Frac<NM> &b) {
@@ -329,7 +338,7 @@ __device__ __forceinline__ double E_of(const MSt<NM> &z) {
 }
 template <int NM>
 __device__ __forceinline__ double alpha(const MSt<NM> &z, int i) {
-    return isnan(z.r[i]) ? 0.0 : fmax_std(0.0, fmin_std(z.b.f[i] * z.rho / z.r[i], 1.0));
+    return volume_fraction(z.b.f[i], z.rho, z.r[i]);
 }
 template <int NM>
 __device__ __forceinline__ QVd<NM> q_of(const MSt<NM> &z) {
@@ -359,11 +368,11 @@ template <int NM>
 __device__ MSt<NM> state_of_q(const MixD<NM> &mx, const QVd<NM> &q, double P0, double T0, const double *rhos0) {
     MSt<NM> z;
     z.rho = q.a[0];
-    z.vx = q.a[1] / z.rho;
-    z.vy = q.a[2] / z.rho;
+    z.vx = div_z(q.a[1], z.rho);
+    z.vy = div_z(q.a[2], z.rho);
     z.e = q.a[3] / z.rho - 0.5 * (z.vx * z.vx + z.vy * z.vy + 0.0 * 0.0);
 #pragma unroll
-    for (int i = 0; i < NM; ++i) z.b.f[i] = q.a[4 + i] / z.rho;
+    for (int i = 0; i < NM; ++i) z.b.f[i] = div_z(q.a[4 + i], z.rho);
     cutoff(z.b, 1.0e-12);
     normalize(z.b);
     int idx = frac_index(z.b);
@@ -493,7 +502,7 @@ __device__ QVd<NM> hllc(const MixD<NM> &mx, const MSt<NM> &zL, const MSt<NM> &zR
     if (S_R <= 0.0) return f_of(zR);
     double a_L = zL.rho * (S_L - zL.vx);
     double a_R = zR.rho * (S_R - zR.vx);
-    double S_C = (zL.P - zR.P + a_R * zR.vx - a_L * zL.vx) / (a_R - a_L);
+    double S_C = div_z(zL.P - zR.P + a_R * zR.vx - a_L * zL.vx, a_R - a_L);
     if (S_C < S_L) S_C = S_L + 1.0e-9 * fmax_std(c_L, c_R);
     if (S_C > S_R) S_C = S_R - 1.0e-9 * fmax_std(c_L, c_R);
     double rho_sL = a_L / (S_L - S_C);
@@ -534,16 +543,16 @@ struct Wave {
 template <int NM>
 __device__ void wave_config(const MixD<NM> &mx, const QVd<NM> &QL, const QVd<NM> &FL, const QVd<NM> &QR,
                             const QVd<NM> &FR, Wave<NM> &w) {
-    double vLx = QL.a[1] / QL.a[0], vLy = QL.a[2] / QL.a[0];
-    double vRx = QR.a[1] / QR.a[0], vRy = QR.a[2] / QR.a[0];
-    double vLz = 0.0 / QL.a[0], vRz = 0.0 / QR.a[0];
+    double vLx = div_z(QL.a[1], QL.a[0]), vLy = div_z(QL.a[2], QL.a[0]);
+    double vRx = div_z(QR.a[1], QR.a[0]), vRy = div_z(QR.a[2], QR.a[0]);
+    double vLz = div_z(0.0, QL.a[0]), vRz = div_z(0.0, QR.a[0]);
     double e_L = QL.a[3] / QL.a[0] - 0.5 * (vLx * vLx + vLy * vLy + vLz * vLz);
     double e_R = QR.a[3] / QR.a[0] - 0.5 * (vRx * vRx + vRy * vRy + vRz * vRz);
     Frac<NM> bL, bR;
 #pragma unroll
     for (int i = 0; i < NM; ++i) {
-        bL.f[i] = QL.a[4 + i] / QL.a[0];
-        bR.f[i] = QR.a[4 + i] / QR.a[0];
+        bL.f[i] = div_z(QL.a[4 + i], QL.a[0]);
+        bR.f[i] = div_z(QR.a[4 + i], QR.a[0]);
     }
     double c_L = sound_speed_re(mx, QL.a[0], e_L, bL);
     double c_R = sound_speed_re(mx, QR.a[0], e_R, bR);
@@ -559,7 +568,7 @@ __device__ void wave_config(const MixD<NM> &mx, const QVd<NM> &QL, const QVd<NM>
         aL.a[k] = FL.a[k] - S_L * QL.a[k];
         aR.a[k] = FR.a[k] - S_R * QR.a[k];
     }
-    double S_C = (aR.a[1] - aL.a[1]) / (aR.a[0] - aL.a[0]);
+    double S_C = div_z(aR.a[1] - aL.a[1], aR.a[0] - aL.a[0]);
     if (S_C < S_L) S_C = S_L + 1.0e-9 * fmax_std(c_L, c_R);
     if (S_C > S_R) S_C = S_R - 1.0e-9 * fmax_std(c_L, c_R);
     double rho_sL = aL.a[0] / (S_C - S_L);

@@ -38,7 +38,7 @@ __device__ __forceinline__ double alpha_rt(const MSt<NM> &z, int idx) {
             r = z.r[i];
             b = z.b.f[i];
         }
-    return isnan(r) ? 0.0 : fmax_std(0.0, fmin_std(b * z.rho / r, 1.0));
+    return volume_fraction(b, z.rho, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(BLOCK) k_recover(MmArgs a) {
 #pragma unroll
             for (int i = 0; i < NM; ++i) {
                 if (ac[i] > 0.0) {
-                    double a_n = isnan(zn.r[i]) ? 0.0 : fmax_std(0.0, fmin_std(zn.b.f[i] * zn.rho / zn.r[i], 1.0));
+                    double a_n = volume_fraction(zn.b.f[i], zn.rho, zn.r[i]);
                     double ff = face_fraction(ac[i], a_n);
                     nx[i] = nx[i] - ff * Sx;
                     ny[i] = ny[i] - ff * Sy;
@@ -158,7 +158,7 @@ __device__ __forceinline__ int master_component(const MSt<NM> &zm, const MSt<NM>
 #pragma unroll
     for (int i = 0; i < NM; ++i) {
         if (w.b.f[i] > 0.0) {
-            double al = isnan(w.r[i]) ? 0.0 : fmax_std(0.0, fmin_std(w.b.f[i] * w.rho / w.r[i], 1.0));
+            double al = volume_fraction(w.b.f[i], w.rho, w.r[i]);
             if (al > alpha_max) {
                 alpha_max = al;
                 master = i;

@@ -107,7 +107,9 @@ __device__ void hllc_pure(const MixD<NM> &mx, const PureSt<R> &zL, const PureSt<
     }
     R a_L = zL.rho * (S_L - zL.vx);
     R a_R = zR.rho * (S_R - zR.vx);
-    R S_C = (zL.P - zR.P + a_R * zR.vx - a_L * zL.vx) / (a_R - a_L);
+    R S_C;
+    if constexpr (sizeof(R) == 8) S_C = div_z(zL.P - zR.P + a_R * zR.vx - a_L * zL.vx, a_R - a_L);
+    else S_C = (zL.P - zR.P + a_R * zR.vx - a_L * zL.vx) / (a_R - a_L);
     if (S_C < S_L) S_C = S_L + R(1.0e-9) * rmax<R>(c_L, c_R);
     if (S_C > S_R) S_C = S_R - R(1.0e-9) * rmax<R>(c_L, c_R);
     R rho_sL = a_L / (S_L - S_C);
@@ -249,11 +251,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_flux_pure(MmArgs a) {
     // mixed results go to the closure list
     MSt<NM> z;
     z.rho = q.a[0];
-    z.vx = q.a[1] / z.rho;
-    z.vy = q.a[2] / z.rho;
+    z.vx = div_z(q.a[1], z.rho);
+    z.vy = div_z(q.a[2], z.rho);
     z.e = q.a[3] / z.rho - 0.5 * (z.vx * z.vx + z.vy * z.vy + 0.0 * 0.0);
 #pragma unroll
-    for (int i = 0; i < NM; ++i) z.b.f[i] = q.a[4 + i] / z.rho;
+    for (int i = 0; i < NM; ++i) z.b.f[i] = div_z(q.a[4 + i], z.rho);
     cutoff(z.b, 1.0e-12);
     normalize(z.b);
     int idx = frac_index(z.b);

@@ -46,6 +46,22 @@ __host__ __device__ inline T smin_t(T a, T b) { return (b < a) ? b : a; }
 template <typename T>
 __host__ __device__ inline T smax_t(T a, T b) { return (a < b) ? b : a; }
 
+// a / b where a is often exactly zero (velocities of a gas at rest, fractions of
+// an absent material, a contact's pressure jump): CUDA's division takes a call
+// out of line for the whole warp when a lane's numerator is zero or its result
+// is not a normal number.  The zero is taken around the division; the result
+// is a / b up to the sign of a zero (NaN for b = 0 or NaN).
+__host__ __device__ inline double div_z(double a, double b) {
+    const bool z = a == 0.0;
+    const double q = (z ? 0x1p-100 : a) / b;
+    return z ? q * 0.0 : q;
+}
+// both non-zero and of one sign (false with a NaN)
+template <typename T>
+__host__ __device__ inline bool same_sign(T a, T b) {
+    return (a > T(0) && b > T(0)) || (a < T(0) && b < T(0));
+}
+
 // Correctly rounded x^3 (stands in for glibc pow(x, 3) in gradient.h:256):
 // Dekker/Knuth error-free products give x^3 = q + qe + pe*x exactly, and the
 // final sum rounds once.  Exact whenever x^3 is representable.
@@ -99,8 +115,8 @@ __host__ __device__ inline Cons q_from_p(const Prim &z) {
 __host__ __device__ inline Prim p_from_q(const Cons &q, const EosD &eos) {
     Prim z;
     z.r = q.r;
-    z.u = q.mu / z.r;
-    z.v = q.mv / z.r;
+    z.u = div_z(q.mu, z.r);
+    z.v = div_z(q.mv, z.r);
     z.e = q.E / z.r - 0.5 * v2(z);
     z.p = eos.pressure_re(z.r, z.e);
     return z;
@@ -147,7 +163,7 @@ __device__ inline Cons hllc(const Prim &zL, const Prim &zR, const EosD &eos) {
 
     double a_L = zL.r * (S_L - zL.u);
     double a_R = zR.r * (S_R - zR.u);
-    double S_C = (zL.p - zR.p + a_R * zR.u - a_L * zL.u) / (a_R - a_L);
+    double S_C = div_z(zL.p - zR.p + a_R * zR.u - a_L * zL.u, a_R - a_L);
     double rho_sL = a_L / (S_L - S_C);
     double rho_sR = a_R / (S_R - S_C);
     double EL = zL.e + 0.5 * v2(zL);
@@ -529,7 +545,10 @@ __device__ inline Cons flux_fx(int kind, const Prim &zL, const Prim &zR, const E
     else return num_flux(kind, zL, zR, eos);
 }
 
-// limiter.cxx binary forms phi(a, b)
+// limiter.cxx binary forms phi(a, b).  Every use multiplies phi by b, and the
+// forms written with r = a / b are 0 for r <= 0 or NaN and finite for b = 0, so
+// they are formed only for two non-zero arguments of one sign: over constant
+// regions the division would leave its short path.
 __device__ inline double lim_MC1(double r) {
     if (isnan(r)) return 0.0;
     return smax(0.0, smin(2 * r, smin(0.5 * (1.0 + r), 2.0)));
@@ -541,7 +560,7 @@ __device__ inline double limiter2(int kind, double a, double b) {
         case LIM_MINMOD:
             if (a * b <= 0.0) return 0.0;
             return smin(a / b, 1.0);
-        case LIM_MC: return lim_MC1(a / b);
+        case LIM_MC: return same_sign(a, b) ? lim_MC1(a / b) : 0.0;
         case LIM_VANLEER:
             if (a * b < 0.0) return 0.0;
             if (a == 0.0) return 0.0;
@@ -567,16 +586,19 @@ __device__ inline double limiter2(int kind, double a, double b) {
             if (a * b <= 0.0) return 0.0;
             return (4.0 * a) / (a + 3.0 * b);
         case LIM_KOREN: {
+            if (!same_sign(a, b)) return 0.0;
             double r = a / b;
             if (isnan(r)) return 0.0;
             return smax(0.0, smin(2 * r, smin(2.0, (1 + 2 * r) / 3.0)));
         }
         case LIM_SMART: {
+            if (!same_sign(a, b)) return 0.0;
             double r = a / b;
             if (isnan(r)) return 0.0;
             return smax(0.0, smin(2.0 * r, smin(0.25 + 0.75 * r, 4.0)));
         }
         case LIM_SUPERBEE: {
+            if (!same_sign(a, b)) return 0.0;
             double r = a / b;
             if (isnan(r)) return 0.0;
             return smax(0.0, smin(smin(2 * r, 1.0), smin(r, 2.0)));

@@ -169,6 +169,7 @@ __device__ inline R lim2(int kind, R a, R b) {
             if (a * b <= R(0)) return R(0);
             return smin_t(a / b, R(1));
         case LIM_MC: {
+            if (!same_sign(a, b)) return R(0);  // (see limiter2)
             R r = a / b;
             if (isnan(r)) return R(0);
             return smax_t(R(0), smin_t(R(2) * r, smin_t(R(0.5) * (R(1) + r), R(2))));
@@ -197,16 +198,19 @@ __device__ inline R lim2(int kind, R a, R b) {
             if (a * b <= R(0)) return R(0);
             return (R(4) * a) / (a + R(3) * b);
         case LIM_KOREN: {
+            if (!same_sign(a, b)) return R(0);  // (see limiter2)
             R r = a / b;
             if (isnan(r)) return R(0);
             return smax_t(R(0), smin_t(R(2) * r, smin_t(R(2), (R(1) + R(2) * r) / R(3))));
         }
         case LIM_SMART: {
+            if (!same_sign(a, b)) return R(0);  // (see limiter2)
             R r = a / b;
             if (isnan(r)) return R(0);
             return smax_t(R(0), smin_t(R(2) * r, smin_t(R(0.25) + R(0.75) * r, R(4))));
         }
         case LIM_SUPERBEE: {
+            if (!same_sign(a, b)) return R(0);  // (see limiter2)
             R r = a / b;
             if (isnan(r)) return R(0);
             return smax_t(R(0), smin_t(smin_t(R(2) * r, R(1)), smin_t(r, R(2))));
