@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -72,16 +73,22 @@ def _stale(target: Path, deps) -> bool:
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
     headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "zephyr_gpu.h"]
-    objs = []
+    objs, todo = [], []
     for unit, extra in UNITS.items():
         src = CSRC / unit
         obj = BUILD / (unit + ".o")
         objs.append(obj)
         if force or _stale(obj, [src, *headers, Path(__file__)]):
-            cmd = [nvcc(), *ARCH, *COMMON, *extra, "-c", str(src), "-o", str(obj)]
-            if verbose:
-                print(" ".join(cmd), flush=True)
-            subprocess.run(cmd, check=True)
+            todo.append([nvcc(), *ARCH, *COMMON, *extra, "-c", str(src), "-o", str(obj)])
+
+    def compile_unit(cmd):
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.run(cmd, check=True)
+
+    # the units are independent: one compiler per core
+    with ThreadPoolExecutor(max_workers=max(1, min(len(todo), os.cpu_count() or 1))) as pool:
+        list(pool.map(compile_unit, todo))
     if force or _stale(OUT, objs):
         cmd = [nvcc(), *ARCH, "-shared", "-o", str(OUT), *map(str, objs), "-cudart", "static"]
         if verbose:

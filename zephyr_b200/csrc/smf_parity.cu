@@ -4,6 +4,7 @@
 // for bit with the oracle and the reference.
 #include <cuda_runtime.h>
 
+#include "smf_parity_tile.cuh"
 #include "smf_struct.cuh"
 
 namespace zg {
@@ -32,26 +33,28 @@ void launch_dt(const SmfArgs &a, PrimPtr z, bool slots, void *stream) {
 // The kernels that evaluate face fluxes, instantiated per flux family: HLLC
 // and HLL without the other fluxes' code (the run-time switch over the
 // eight fluxes of NumFlux::create costs registers and spills), the general
-// switch for the rest.  The same operations either way.
+// switch for the rest.  The same operations either way.  On a rectangle the
+// second order with HLLC or HLL runs in the tile kernels.
 template <int FX>
-static void flux1_fx(const SmfArgs &a, bool slots, void *stream) {
-    if (slots) k_flux1<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a);
-    else k_flux1<StructAcc, BLOCK, 1, FX><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a);
+static void flux1_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
+    if (slots) k_flux1<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
+    else k_flux1<StructAcc, BLOCK, 1, FX><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
 }
 template <int FX>
-static void stage2_fx(const SmfArgs &a, bool slots, void *stream) {
-    if (slots) k_stage2<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a);
-    else k_stage2<StructAcc, BLOCK, 1, FX><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a);
+static void stage2_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
+    if (slots) k_stage2<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
+    else k_stage2<StructAcc, BLOCK, 1, -1><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
 }
 template <int FX>
-static void heun_fx(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, bool slots, void *stream) {
+static void heun_fx(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, double *dt_next, bool slots,
+                    void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (slots) {
-        if (final) k_heun<SlotAcc, BLOCK, true, 1, FX><<<blocks(a, true), BLOCK, 0, st>>>(a, zin, zout);
+        if (final) k_heun<SlotAcc, BLOCK, true, 1, FX><<<blocks(a, true), BLOCK, 0, st>>>(a, zin, zout, dt_next);
         else k_heun<SlotAcc, BLOCK, false, 1, FX><<<blocks(a, true), BLOCK, 0, st>>>(a, zin, zout);
     } else {
-        if (final) k_heun<StructAcc, BLOCK, true, 1, FX><<<blocks(a, false), BLOCK, 0, st>>>(a, zin, zout);
-        else k_heun<StructAcc, BLOCK, false, 1, FX><<<blocks(a, false), BLOCK, 0, st>>>(a, zin, zout);
+        if (final) k_heun<StructAcc, BLOCK, true, 1, -1><<<blocks(a, false), BLOCK, 0, st>>>(a, zin, zout, dt_next);
+        else k_heun<StructAcc, BLOCK, false, 1, -1><<<blocks(a, false), BLOCK, 0, st>>>(a, zin, zout);
     }
 }
 #define ZG_FLUX_FAMILY(FN, ...)                                        \
@@ -61,12 +64,46 @@ static void heun_fx(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, boo
         else FN<-1>(__VA_ARGS__);                                      \
     } while (0)
 
-void launch_flux1(const SmfArgs &a, bool slots, void *stream) { ZG_FLUX_FAMILY(flux1_fx, a, slots, stream); }
+void launch_flux1(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
+    ZG_FLUX_FAMILY(flux1_fx, a, dt_next, slots, stream);
+}
 void launch_grad(const SmfArgs &a, PrimPtr z, bool slots, void *stream) { ZG_DISPATCH(k_grad, a, z); }
 void launch_stage1(const SmfArgs &a, bool slots, void *stream) { ZG_DISPATCH(k_stage1, a); }
-void launch_stage2(const SmfArgs &a, bool slots, void *stream) { ZG_FLUX_FAMILY(stage2_fx, a, slots, stream); }
-void launch_heun(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, bool slots, void *stream) {
-    ZG_FLUX_FAMILY(heun_fx, a, zin, zout, final, slots, stream);
+void launch_stage2(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
+    ZG_FLUX_FAMILY(stage2_fx, a, dt_next, slots, stream);
+}
+void launch_heun(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, double *dt_next, bool slots, void *stream) {
+    ZG_FLUX_FAMILY(heun_fx, a, zin, zout, final, dt_next, slots, stream);
+}
+
+// Rows of a tile and blocks per SM of the tile kernels (smf_parity_tile.cuh).
+#ifndef ZG_PTILE_TH
+#define ZG_PTILE_TH 12
+#endif
+#ifndef ZG_PTILE_MINB
+#define ZG_PTILE_MINB 2
+#endif
+template <int MODE, int LIM>
+static void tile_flux(const ptile::Args &A, cudaStream_t s) {
+    if (A.a.flux == FLUX_HLL) ptile::launch<MODE, LIM, true, ZG_PTILE_TH, ZG_PTILE_MINB>(A, s);
+    else ptile::launch<MODE, LIM, false, ZG_PTILE_TH, ZG_PTILE_MINB>(A, s);
+}
+template <int MODE>
+static void tile_lim(const ptile::Args &A, cudaStream_t s) {
+    switch (A.a.limiter) {  // the common limiters are compiled in
+        case LIM_VANALBADA1: tile_flux<MODE, LIM_VANALBADA1>(A, s); break;
+        case LIM_MC: tile_flux<MODE, LIM_MC>(A, s); break;
+        case LIM_MINMOD: tile_flux<MODE, LIM_MINMOD>(A, s); break;
+        default: tile_flux<MODE, -1>(A, s); break;
+    }
+}
+void launch_tile(const SmfArgs &a, const ptile::Axis &x, const ptile::Axis &y, int stage, PrimPtr zin, PrimPtr zout,
+                 const double *dt_in, double *dt_next, void *stream) {
+    const ptile::Args A{a, x, y, zin, zout, dt_in, dt_next};
+    const cudaStream_t s = (cudaStream_t)stream;
+    if (stage == ptile::PC) tile_lim<ptile::PC>(A, s);
+    else if (stage == ptile::HEUN_A) tile_lim<ptile::HEUN_A>(A, s);
+    else tile_lim<ptile::HEUN_B>(A, s);
 }
 void launch_flags(const SmfArgs &a, int *flags, bool slots, void *stream) { ZG_DISPATCH(k_flags, a, flags); }
 

@@ -59,15 +59,35 @@ struct SmfArgs {
     double *dt_out;                 // dt of the current step, written by the dt kernel
 };
 
+// Per-axis geometry of the PARITY tile kernels (smf_parity_tile.cuh), per cell
+// index: weight and offset of the low and high neighbour (gradient.h:251-258;
+// the normal projection equals the offset on an axis-aligned rectangle), the
+// least-squares diagonal, the offsets of the low and high face and of the other
+// axis' faces from the centre; and the offsets of the two faces of a periodic
+// seam from the mirrored centres (sm_fluid.cpp:308-322).
+namespace ptile {
+struct Axis {
+    const double *wl, *rl, *wh, *rh, *A, *ol, *oh, *om;
+    double seam_lo, seam_hi;
+};
+enum : int { PC = 1, HEUN_A = 2, HEUN_B = 3 };
+}  // namespace ptile
+
 // Launchers (one set per numerics flavour).
 // Parity kernels; `slots` selects the slot-mesh (AMR) geometry.
 namespace parity {
+// One second-order stage (ptile::PC ... HEUN_B) of a rectangle with HLLC or HLL in one
+// kernel: zin -> zout at the dt in *dt_in; the last stage leaves the next dt
+// in *dt_next.
+void launch_tile(const SmfArgs &a, const ptile::Axis &x, const ptile::Axis &y, int stage, PrimPtr zin, PrimPtr zout,
+                 const double *dt_in, double *dt_next, void *stream);
 void launch_dt(const SmfArgs &a, PrimPtr z, bool slots, void *stream);
-void launch_flux1(const SmfArgs &a, bool slots, void *stream);
+// dt_next (the last kernel of a step): the next step's dt goes there
+void launch_flux1(const SmfArgs &a, double *dt_next, bool slots, void *stream);
 void launch_grad(const SmfArgs &a, PrimPtr z, bool slots, void *stream);
 void launch_stage1(const SmfArgs &a, bool slots, void *stream);
-void launch_stage2(const SmfArgs &a, bool slots, void *stream);
-void launch_heun(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, bool slots, void *stream);
+void launch_stage2(const SmfArgs &a, double *dt_next, bool slots, void *stream);
+void launch_heun(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, double *dt_next, bool slots, void *stream);
 void launch_flags(const SmfArgs &a, int *flags, bool slots, void *stream);
 }  // namespace parity
 

@@ -57,6 +57,8 @@ struct zg_ctx {
     double *d_tgeo = nullptr;  // per-axis tables of the tiled kernels, FP64 then FP32
     tiled::AxisGeo<double> ax64{}, ay64{};
     tiled::AxisGeo<float> ax32{}, ay32{};
+    double *d_pgeo = nullptr;  // per-axis tables of the PARITY tile kernels
+    ptile::Axis pax{}, pay{};
     int cap = 0;  // cells every per-cell field holds (n, or the adaptive mesh's capacity)
 
     // adaptive mesh (AmrCells layout on the device)
@@ -92,7 +94,7 @@ struct zg_ctx {
     unsigned int *d_ticket = nullptr;
     double *d_dt = nullptr;     // dt of the last step
     double *d_dt2 = nullptr;    // the other dt slot: the next step's dt when dt_next_ready
-    bool dt_next_ready = false; // the FAST adaptive step's cell sums left the next dt in d_dt2
+    bool dt_next_ready = false; // the last step (FAST adaptive, PARITY) left the next dt in d_dt2
     int *d_flags = nullptr;
     PrimPtr z{}, zhalf{}, znext{};
     double *gx[4] = {}, *gy[4] = {};
@@ -224,6 +226,7 @@ void free_solver(zg_ctx *c) {
 void free_mesh(zg_ctx *c) {
     cudaFree(c->d_geo);
     cudaFree(c->d_tgeo);
+    cudaFree(c->d_pgeo);
     cudaFree(c->d_slot);
     cudaFree(c->d_axial);
     c->d_axial = nullptr;
@@ -238,6 +241,7 @@ void free_mesh(zg_ctx *c) {
     if (c->state_mode == STATE_ORDERED_MIXED) c->state_mode = ZG_MIXED;
     c->d_geo = nullptr;
     c->d_tgeo = nullptr;
+    c->d_pgeo = nullptr;
     c->d_slot = nullptr;
     c->d_amr = nullptr;
     c->d_amr_scratch = nullptr;
@@ -460,6 +464,41 @@ std::vector<double> axis_tables(const std::vector<double> &V, const std::vector<
     return t;
 }
 
+// Tables of ptile::Axis for one axis, with the gather kernels' expressions
+// (lsm_limited, neib_center, extrap in smf_struct.cuh) term by term; the same
+// arguments as axis_tables.  Eight tables of n values.
+std::vector<double> parity_tables(const std::vector<double> &V, const std::vector<double> &C,
+                                  const std::vector<double> &M, double area, double seam[2]) {
+    const int n = (int)C.size();
+    std::vector<double> t(8 * (size_t)n);
+    for (int i = 0; i < n; ++i) {
+        double wr[2], A = 0.0;
+        for (int side = 0; side < 2; ++side) {
+            const bool inner = side == 0 ? i > 0 : i < n - 1;
+            const double fc = side == 0 ? V[i] : V[i + 1], nrm = side == 0 ? -1.0 : 1.0;
+            double nc;
+            if (inner) {
+                nc = side == 0 ? C[i - 1] : C[i + 1];
+            } else {  // mirror of the centre in the face (amr_faces.h:197-199)
+                const double d = (fc - C[i]) * nrm, two = 2.0 * d;
+                nc = C[i] + two * nrm;
+                seam[side] = fc - nc;
+            }
+            const double r = nc - C[i];
+            const double w = area / cube_rn(std::sqrt(r * r));
+            wr[side] = w * r;
+            A += wr[side] * r;
+            t[(size_t)(2 * side) * n + i] = w;
+            t[(size_t)(2 * side + 1) * n + i] = r;
+        }
+        t[(size_t)4 * n + i] = A;
+        t[(size_t)5 * n + i] = V[i] - C[i];
+        t[(size_t)6 * n + i] = V[i + 1] - C[i];
+        t[(size_t)7 * n + i] = M[i] - C[i];
+    }
+    return t;
+}
+
 std::string lower_strip(const char *name) {
     std::string s;
     for (const char *p = name; *p; ++p) s.push_back((char)std::tolower((unsigned char)*p));
@@ -540,28 +579,49 @@ int ensure_side(zg_ctx *c) {
     return ZG_OK;
 }
 
-// One step of SmFluid::update (sm_fluid.cpp:81-102) as kernel launches.
+// PARITY steps that run in the tile kernels: the second order of a rectangle
+// with HLLC or HLL.
+bool parity_tiles(const zg_ctx *c) {
+    return !c->slots && c->par.accuracy == 2 && (c->par.flux == ZG_FLUX_HLLC || c->par.flux == ZG_FLUX_HLL);
+}
+
+// One step of SmFluid::update (sm_fluid.cpp:81-102) as kernel launches, bit
+// for bit.  The step's last kernel also takes the dt of the state it writes,
+// into the other dt slot; a dt pass runs only after the state came from
+// elsewhere.
 int enqueue_parity_step(zg_ctx *c) {
     if (c->par.accuracy == 2) c->grad_ordered = false;  // this step's gradients, in the mesh's order
-    SmfArgs a = make_args(c);
     void *st = (void *)c->stream;
-    timed(c, ZG_K_DT, [&] { parity::launch_dt(a, c->z, c->slots, st); });
+    const bool have_dt = c->dt_next_ready, pc = c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR;
+    if (have_dt) std::swap(c->d_dt, c->d_dt2);
+    SmfArgs a = make_args(c);
+    if (!have_dt) timed(c, ZG_K_DT, [&] { parity::launch_dt(a, c->z, c->slots, st); });
+    double *next = c->d_dt2;
+    auto tile = [&](int kind, int stage, PrimPtr zin, PrimPtr zout) {
+        timed(c, kind, [&] { parity::launch_tile(a, c->pax, c->pay, stage, zin, zout, c->d_dt, next, st); });
+    };
     if (c->par.accuracy == 1) {
-        timed(c, ZG_K_FLUX1, [&] { parity::launch_flux1(a, c->slots, st); });
-    } else if (c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR) {
+        timed(c, ZG_K_FLUX1, [&] { parity::launch_flux1(a, next, c->slots, st); });
+    } else if (parity_tiles(c) && pc) {
+        tile(ZG_K_STEP, ptile::PC, c->z, c->znext);
+    } else if (parity_tiles(c)) {
+        tile(ZG_K_HEUN_A, ptile::HEUN_A, c->z, c->zhalf);
+        tile(ZG_K_HEUN_B, ptile::HEUN_B, c->zhalf, c->znext);
+    } else if (pc) {
         timed(c, ZG_K_GRAD, [&] { parity::launch_grad(a, c->z, c->slots, st); });
         timed(c, ZG_K_STAGE1, [&] { parity::launch_stage1(a, c->slots, st); });
-        timed(c, ZG_K_STAGE2, [&] { parity::launch_stage2(a, c->slots, st); });
-        c->wait_cur = 1 - c->wait_cur;
+        timed(c, ZG_K_STAGE2, [&] { parity::launch_stage2(a, next, c->slots, st); });
     } else {
         timed(c, ZG_K_GRAD, [&] { parity::launch_grad(a, c->z, c->slots, st); });
-        timed(c, ZG_K_HEUN_A, [&] { parity::launch_heun(a, c->z, c->zhalf, false, c->slots, st); });
+        timed(c, ZG_K_HEUN_A, [&] { parity::launch_heun(a, c->z, c->zhalf, false, nullptr, c->slots, st); });
         timed(c, ZG_K_GRAD, [&] { parity::launch_grad(a, c->zhalf, c->slots, st); });
-        timed(c, ZG_K_HEUN_B, [&] { parity::launch_heun(a, c->zhalf, c->znext, true, c->slots, st); });
+        timed(c, ZG_K_HEUN_B, [&] { parity::launch_heun(a, c->zhalf, c->znext, true, next, c->slots, st); });
     }
+    if (c->par.accuracy == 2 && pc) c->wait_cur = 1 - c->wait_cur;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "kernel launch");
     std::swap(c->z, c->znext);  // Storage::swap of init and next (sm_fluid.cpp:368-370)
+    c->dt_next_ready = true;
     c->cfl_valid = false;
     c->stepped = true;
     return ZG_OK;
@@ -854,6 +914,8 @@ int enqueue_step(zg_ctx *c) {
         if (rc != ZG_OK) return rc;
         return enqueue_tiled_step<float, true>(c);
     }
+    // (convert_state forgets the next dt: the state may have changed; here it has not)
+    if (!fast && c->state_mode == ZG_FP64) return enqueue_parity_step(c);
     int rc = convert_state(c, ZG_FP64);
     if (rc != ZG_OK) return rc;
     if (fast) return enqueue_tiled_step<double, false>(c);
@@ -1026,6 +1088,22 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
         fill(c->ay64, c->d_tgeo + tx.size(), ny);
         fill(c->ax32, f32, nx);
         fill(c->ay32, f32 + tx.size(), ny);
+    }
+
+    // per-axis tables of the PARITY tile kernels
+    {
+        double sx[2], sy[2];
+        std::vector<double> t = parity_tables(X, cx, fxm, (y_max - y_min) / ny, sx);
+        const std::vector<double> ty = parity_tables(Y, cy, fym, (x_max - x_min) / nx, sy);
+        t.insert(t.end(), ty.begin(), ty.end());
+        ZG_CUDA(c, cudaMalloc(&c->d_pgeo, t.size() * sizeof(double)));
+        ZG_CUDA(c, cudaMemcpy(c->d_pgeo, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+        auto axis = [](const double *b, size_t n, const double seam[2]) {
+            return ptile::Axis{b,         b + n,     b + 2 * n, b + 3 * n, b + 4 * n,
+                               b + 5 * n, b + 6 * n, b + 7 * n, seam[0],   seam[1]};
+        };
+        c->pax = axis(c->d_pgeo, (size_t)nx, sx);
+        c->pay = axis(c->d_pgeo + 8 * (size_t)nx, (size_t)ny, sy);
     }
 
     StructMesh &m = c->mesh;
@@ -2676,8 +2754,10 @@ int zg_amr_enable(zg_ctx *c, int max_level, int capacity) {
     // the rectangle's axis tables are not used on a slot mesh
     cudaFree(c->d_geo);
     cudaFree(c->d_tgeo);
+    cudaFree(c->d_pgeo);
     c->d_geo = nullptr;
     c->d_tgeo = nullptr;
+    c->d_pgeo = nullptr;
     c->ax64 = c->ay64 = tiled::AxisGeo<double>{};
     c->ax32 = c->ay32 = tiled::AxisGeo<float>{};
     c->cap = capacity;

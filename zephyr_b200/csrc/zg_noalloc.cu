@@ -177,7 +177,7 @@ extern "C" int zg_rect_step_noalloc(int device, int nx, int ny, double x_min, do
     if (cudaGetLastError() != cudaSuccess) return ZG_ERR_CUDA;
     parity::launch_dt(a, a.z, false, stream);
     if (cudaGetLastError() != cudaSuccess) return ZG_ERR_CUDA;
-    parity::launch_flux1(a, false, stream);
+    parity::launch_flux1(a, nullptr, false, stream);
     if (cudaGetLastError() != cudaSuccess) return ZG_ERR_CUDA;
     if (dt && cudaMemcpyAsync(dt, s + 2, sizeof(double), cudaMemcpyDefault, st) != cudaSuccess)
         return ZG_ERR_CUDA;
