@@ -56,12 +56,6 @@ constexpr int BLOCK = 128;
 // bound; these caps on their registers (a few spilled bytes in some) were
 // chosen by timing the 1024^2, 100-step forward and gradient runs over a
 // sweep of the values on a B200 (-D overrides).
-#ifndef ZG_ADJ_PG_MINB
-#define ZG_ADJ_PG_MINB 8
-#endif
-#ifndef ZG_ADJ_FU_MINB
-#define ZG_ADJ_FU_MINB 6
-#endif
 #ifndef ZG_ADJ_VF_MINB
 #define ZG_ADJ_VF_MINB 6
 #endif
@@ -69,6 +63,7 @@ constexpr int BLOCK = 128;
 struct Grid {
     int nx, ny, n;
     double hx, hy, vol;
+    double i2x, i2y;  // 1 / 2h per axis
     double x0, y0;
 };
 // four field arrays of element type S (FP64 state, adjoint and primitive
@@ -128,29 +123,6 @@ __global__ void k_init(Grid g, CF4 W0, double gamma, F4 U) {
     U.f[3][ic] = p / (gamma - 1.0) + 0.5 * (r * (u * u + v * v));
 }
 
-// primitive state and limited slopes of every cell: the primitive map and
-// the neighbour differences in FP64, the slopes from the differences in S
-template <class S>
-__global__ void __launch_bounds__(BLOCK, ZG_ADJ_PG_MINB) k_prim_grad(Grid g, CF4 U, double gamma, double eps,
-                                                                     F4 W, F4T<S> gx, F4T<S> gy) {
-    int ic = blockIdx.x * BLOCK + threadIdx.x;
-    if (ic >= g.n) return;
-    double wc[4], wl[4], wr[4], wb[4], wt[4];
-    prim_at(U, ic, gamma, wc);
-    const Cell c = cell_of(g, ic);
-    prim_at(U, xm(g, c).ic, gamma, wl);
-    prim_at(U, xp(g, c).ic, gamma, wr);
-    prim_at(U, ym(g, c).ic, gamma, wb);
-    prim_at(U, yp(g, c).ic, gamma, wt);
-    const S i2x = S(0.5 / g.hx), i2y = S(0.5 / g.hy), e = S(eps);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        W.f[k][ic] = wc[k];
-        gx.f[k][ic] = slope<S>(S(wl[k] - wc[k]), S(wr[k] - wc[k]), i2x, e);
-        gy.f[k][ic] = slope<S>(S(wb[k] - wc[k]), S(wt[k] - wc[k]), i2y, e);
-    }
-}
-
 // Face states of the face between `lo` and `hi` along an axis, in the face
 // frame (x faces: (rho, u, v, p); y faces: (rho, v, -u, p)): the FP64
 // primitive state rounded to S, plus or minus the slope times h / 2 in S.
@@ -174,72 +146,101 @@ __device__ __forceinline__ void face_states(const CF4 &W, const CF4T<S> &G, int 
         R[0] = b[0]; R[1] = b[2]; R[2] = -b[1]; R[3] = b[3];
     }
 }
-// face-frame flux back to the global frame
+// One Heun stage in one kernel: out = alpha * base + beta * (X + dt L(X)).  A
+// block holds a tile of 30 x STH cells with its two-cell halo in shared memory:
+// primitive states (FP64), slopes (S, from FP64 differences), every face flux of
+// the tile once (FP64: FP32 fluxes carry rounding errors of ~1e-7 of the flux,
+// ~1e-4 of the flux difference across a cell of a smooth field, and the
+// limiter's partials, which depend on neighbour differences, carry that noise
+// of the trajectory into the gradient), then the update.  With `keep` the
+// primitive states and slopes also go to memory, for the reverse sweep.
+//
+// The two kernels it replaces (primitive states and slopes of every cell to
+// memory; fluxes from both sides of every face, IEEE divisions, the symmetric
+// HLLC) took 41 + 103 us a stage at 1024^2, 74M instructions and 244 MB; this one
+// 73 us, 32M instructions and 128 MB.  The 1024^2, 100-step gradient: 82.1 -> 51.1
+// ms, of which the one-sided reverse (adj_math.cuh: k_vjp_faces 94 -> 63 us) 6 ms.
+constexpr int STH = 14;
 template <class S>
-__device__ __forceinline__ void flux_global(const S Fl[4], bool yface, S F[4]) {
-    if (!yface) {
+struct StageShm {
+    double W[4][STH + 4][34];
+    double FX[4][STH + 1][32], FY[4][STH][32];
+    S G[8][STH + 2][32];
+};
+__device__ __forceinline__ int wrapc(int x, int n);
+template <class S>
+__global__ void __launch_bounds__(32 * (STH + 2), 2) k_stage(Grid g, CF4 X, double gamma, double igm1, double eps,
+                                                             CF4 base, double alpha, double beta, double c, bool keep,
+                                                             F4 Wout, F4T<S> gx, F4T<S> gy, F4 out) {
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    StageShm<S> &sm = *reinterpret_cast<StageShm<S> *>(stage_smem);
+    const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l;
+    const int i0 = blockIdx.y * STH, j0 = blockIdx.x * 30;
+    for (int k = tid; k < (STH + 4) * 34; k += 32 * (STH + 2)) {
+        const int zr = k / 34, zc = k - zr * 34;
+        double w[4];
+        prim_at(X, wrapc(i0 + zr - 2, g.nx) * g.ny + wrapc(j0 + zc - 2, g.ny), gamma, w);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) F[k] = Fl[k];
-    } else {
-        F[0] = Fl[0];
-        F[1] = -Fl[2];
-        F[2] = Fl[1];
-        F[3] = Fl[3];
+        for (int q = 0; q < 4; ++q) sm.W[q][zr][zc] = w[q];
     }
-}
-
-// out = alpha * base + beta * (X + dt L(X)), L from the face fluxes of W, G
-template <class S>
-__global__ void __launch_bounds__(BLOCK, ZG_ADJ_FU_MINB) k_flux_update(Grid g, CF4 W, CF4T<S> gx, CF4T<S> gy,
-                                                                       double gamma, CF4 X, CF4 base, double alpha,
-                                                                       double beta, double dt, F4 out) {
-    int ic = blockIdx.x * BLOCK + threadIdx.x;
-    if (ic >= g.n) return;
-    const Cell cc = cell_of(g, ic);
-    const int nb[4] = {xm(g, cc).ic, xp(g, cc).ic, ym(g, cc).ic, yp(g, cc).ic};
-    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    __syncthreads();
+    const int i = i0 - 1 + r, j = j0 - 1 + l;  // the thread's cell
+    const bool mine = r >= 1 && r <= STH && l >= 1 && l <= 30 && i < g.nx && j < g.ny;
+    const int ic = i * g.ny + j;
+    {
+        const S i2x = S(g.i2x), i2y = S(g.i2y), e = S(eps);
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const bool yface = s >= 2, high = (s & 1) == 1;
-        const int lo = high ? ic : nb[s], hi = high ? nb[s] : ic;
-        const double half_h = 0.5 * (yface ? g.hy : g.hx), A = yface ? g.hx : g.hy;
-        // face states and HLLC in FP64 in both forms (the slopes are FP32 in
-        // the mixed form): FP32 fluxes carry rounding errors of ~1e-7 of the
-        // flux, ~1e-4 of the flux difference across a cell of a smooth
-        // field, and the limiter's partials, which depend on neighbour
-        // differences, carry that noise of the trajectory into the gradient
-        double L[4], R[4], Fl[4], F[4];
-        {
-            const CF4T<S> &G = yface ? gy : gx;
-            double a_[4], b_[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                a_[k] = W.f[k][lo] + (double)G.f[k][lo] * half_h;
-                b_[k] = W.f[k][hi] - (double)G.f[k][hi] * half_h;
-            }
-            if (!yface) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    L[k] = a_[k];
-                    R[k] = b_[k];
-                }
-            } else {
-                L[0] = a_[0]; L[1] = a_[2]; L[2] = -a_[1]; L[3] = a_[3];
-                R[0] = b_[0]; R[1] = b_[2]; R[2] = -b_[1]; R[3] = b_[3];
+        for (int q = 0; q < 4; ++q) {
+            const double w = sm.W[q][r + 1][l + 1];
+            const S sx = slope<S>(S(sm.W[q][r][l + 1] - w), S(sm.W[q][r + 2][l + 1] - w), i2x, e);
+            const S sy = slope<S>(S(sm.W[q][r + 1][l] - w), S(sm.W[q][r + 1][l + 2] - w), i2y, e);
+            sm.G[q][r][l] = sx;
+            sm.G[4 + q][r][l] = sy;
+            if (keep && mine) {
+                Wout.f[q][ic] = w;
+                gx.f[q][ic] = sx;
+                gy.f[q][ic] = sy;
             }
         }
-        hllc<double>(L, R, gamma, Fl);
-        flux_global<double>(Fl, yface, F);
-        const double sgn = high ? A : -A;  // outward flux of this cell
-#pragma unroll
-        for (int k = 0; k < 4; ++k) sum[k] += sgn * (double)F[k];
     }
-    const double c = dt / g.vol;
+    if (!out.f[0]) return;  // primitive states and slopes only
+    __syncthreads();
+    if (r <= STH && l >= 1 && l <= 30) {  // +x face of cell (r, l)
+        const double h = 0.5 * g.hx;
+        double L[4], R[4], F[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        double v = beta * (X.f[k][ic] - c * sum[k]);
-        if (alpha != 0.0) v += alpha * base.f[k][ic];
-        out.f[k][ic] = v;
+        for (int q = 0; q < 4; ++q) {
+            L[q] = sm.W[q][r + 1][l + 1] + (double)sm.G[q][r][l] * h;
+            R[q] = sm.W[q][r + 2][l + 1] - (double)sm.G[q][r + 1][l] * h;
+        }
+        hllc<double>(L, R, gamma, igm1, F);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sm.FX[q][r][l] = F[q];
+    }
+    if (r >= 1 && r <= STH && l <= 30) {  // +y face: the normal velocity is v
+        const double h = 0.5 * g.hy;
+        double L[4], R[4], F[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int t = q == 1 ? 2 : (q == 2 ? 1 : q);
+            L[t] = sm.W[q][r + 1][l + 1] + (double)sm.G[4 + q][r][l] * h;
+            R[t] = sm.W[q][r + 1][l + 2] - (double)sm.G[4 + q][r][l + 1] * h;
+        }
+        hllc<double>(L, R, gamma, igm1, F);
+        sm.FY[0][r - 1][l] = F[0];
+        sm.FY[1][r - 1][l] = F[2];
+        sm.FY[2][r - 1][l] = F[1];
+        sm.FY[3][r - 1][l] = F[3];
+    }
+    __syncthreads();
+    if (!mine) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double sum =
+            g.hy * (sm.FX[q][r][l] - sm.FX[q][r - 1][l]) + g.hx * (sm.FY[q][r - 1][l] - sm.FY[q][r - 1][l - 1]);
+        double v = beta * (X.f[q][ic] - c * sum);
+        if (alpha != 0.0) v += alpha * base.f[q][ic];
+        out.f[q][ic] = v;
     }
 }
 
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(VJ *VI, ZG_ADJ_VT_MINB) k_vjp_cells_tiled(
     const int tj = threadIdx.x, ti = threadIdx.y, tid = ti * VJ + tj;
     const int i0 = blockIdx.y * VI, j0 = blockIdx.x * VJ;
     const size_t n = (size_t)g.n;
-    const S i2x = S(0.5 / g.hx), i2y = S(0.5 / g.hy), hx2 = S(0.5 * g.hx), hy2 = S(0.5 * g.hy), se = S(eps);
+    const S i2x = S(g.i2x), i2y = S(g.i2y), hx2 = S(0.5 * g.hx), hy2 = S(0.5 * g.hy), se = S(eps);
     const Cell c{wrapc(i0 + ti, g.nx) * g.ny + wrapc(j0 + tj, g.ny), wrapc(i0 + ti, g.nx), wrapc(j0 + tj, g.ny)};
     const Cell cl = xm(g, c), cr = xp(g, c), cb = ym(g, c), ct = yp(g, c);
     const bool live = i0 + ti < g.nx && j0 + tj < g.ny;
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(VJ *VI, ZG_ADJ_VT_MINB) k_vjp_cells_tiled(
         const int ic = c.ic;
         // the primitive map's partials at the stage's primitive state
         // (rho, u, v, p): E - rho |v|^2 / 2 = p / (gamma - 1)
-        const double ir = 1.0 / wc[0], u = wc[1], v = wc[2], gm1 = gamma - 1.0;
+        const double ir = trcp(wc[0]), u = wc[1], v = wc[2], gm1 = gamma - 1.0;
         double ub[4];
         ub[0] = wt[0] - wt[1] * u * ir - wt[2] * v * ir + wt[3] * gm1 * 0.5 * (u * u + v * v);
         ub[1] = wt[1] * ir - wt[3] * gm1 * u;
@@ -538,7 +539,7 @@ struct zg_adj {
     double *d_all = nullptr;
     size_t cap_ckpt = 0, cap_seg = 0;  // checkpoints and segment states held
     double *d_acc = nullptr;           // per-block accumulators: J, gamma
-    F4 U0{}, Ua{}, Ub{}, Ustar{}, W{}, gx{}, gy{}, lamA{}, lamB{}, lamS{};
+    F4 Ua{}, Ub{}, Ustar{}, lamA{}, lamB{}, lamS{};
     double *fbx = nullptr, *fby = nullptr;  // face-state cotangents, 8 n each
     std::vector<F4> ckpt;
     // two sets of segment storage: the states, stage values, primitive states
@@ -588,7 +589,7 @@ int reserve(zg_adj *a, size_t ckpts, size_t seglen) {
     cudaFree(a->d_all);
     a->d_all = nullptr;
     size_t n = (size_t)a->g.n;
-    size_t fields = 10 * 4 + 16 + 4 * ckpts + 2 * (4 * (seglen + 1) + 4 * seglen + 3 * 4 * (2 * seglen));
+    size_t fields = 6 * 4 + 16 + 4 * ckpts + 2 * (4 * (seglen + 1) + 4 * seglen + 3 * 4 * (2 * seglen));
     cudaError_t e = cudaMalloc(&a->d_all, fields * n * sizeof(double));
     if (e != cudaSuccess) return afail(a, ZG_ERR_ALLOC, std::string("adjoint storage: ") + cudaGetErrorString(e));
     double *p = a->d_all;
@@ -600,7 +601,7 @@ int reserve(zg_adj *a, size_t ckpts, size_t seglen) {
         }
         return x;
     };
-    for (F4 *x : {&a->U0, &a->Ua, &a->Ub, &a->Ustar, &a->W, &a->gx, &a->gy, &a->lamA, &a->lamB, &a->lamS})
+    for (F4 *x : {&a->Ua, &a->Ub, &a->Ustar, &a->lamA, &a->lamB, &a->lamS})
         *x = take();
     a->fbx = take().f[0];  // two consecutive groups of 4 n: 8 n
     take();
@@ -650,25 +651,37 @@ CF4T<S> cas(const F4 &x) {
 }
 
 template <class S>
-void heun_step_t(zg_adj *a, cudaStream_t st, const zg_adj_params &p, const F4 &X, const F4 &star, const F4 &out,
-                 const WG &sa, const WG &sb, bool need_out) {
-    unsigned nb = nblocks(a);
-    k_prim_grad<S><<<nb, BLOCK, 0, st>>>(a->g, cf(X), p.gamma, p.limiter_eps, sa.W, as<S>(sa.gx), as<S>(sa.gy));
-    k_flux_update<S><<<nb, BLOCK, 0, st>>>(a->g, cf(sa.W), cas<S>(sa.gx), cas<S>(sa.gy), p.gamma, cf(X), kNull,
-                                           0.0, 1.0, p.dt, star);
-    k_prim_grad<S><<<nb, BLOCK, 0, st>>>(a->g, cf(star), p.gamma, p.limiter_eps, sb.W, as<S>(sb.gx), as<S>(sb.gy));
-    a->launches += 3;
-    if (!need_out) return;
-    k_flux_update<S><<<nb, BLOCK, 0, st>>>(a->g, cf(sb.W), cas<S>(sb.gx), cas<S>(sb.gy), p.gamma, cf(star),
-                                           cf(X), 0.5, 0.5, p.dt, out);
+void stage(zg_adj *a, cudaStream_t st, const zg_adj_params &p, const F4 &X, const CF4 &base, double alpha, double beta,
+           const WG *keep, const F4 &out) {
+    static unsigned long long attr_set = 0;  // devices on which the attribute is set
+    if (a->device >= 64 || !(attr_set >> a->device & 1ull)) {
+        cudaFuncSetAttribute(k_stage<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StageShm<S>));
+        if (a->device < 64) attr_set |= 1ull << a->device;
+    }
+    const WG wg = keep ? *keep : WG{};
+    const dim3 grid((unsigned)((a->g.ny + 29) / 30), (unsigned)((a->g.nx + STH - 1) / STH));
+    k_stage<S><<<grid, dim3(32, STH + 2), sizeof(StageShm<S>), st>>>(
+        a->g, cf(X), p.gamma, 1.0 / (p.gamma - 1.0), p.limiter_eps, base, alpha, beta, p.dt / a->g.vol, keep != nullptr,
+        wg.W, as<S>(wg.gx), as<S>(wg.gy), out);
     ++a->launches;
 }
+// keep: the stages' primitive states and slopes go to sa and sb (else they
+// stay in the kernels)
+template <class S>
+void heun_step_t(zg_adj *a, cudaStream_t st, const zg_adj_params &p, const F4 &X, const F4 &star, const F4 &out,
+                 const WG *sa, const WG *sb, bool need_out) {
+    stage<S>(a, st, p, X, kNull, 0.0, 1.0, sa, star);
+    if (need_out) {
+        stage<S>(a, st, p, star, cf(X), 0.5, 0.5, sb, out);
+    } else if (sb) {  // its primitive states and slopes only, by the same kernel (the same bits)
+        stage<S>(a, st, p, star, kNull, 0.0, 0.0, sb, kNullW);
+    }
+}
 void heun_step(zg_adj *a, cudaStream_t st, const zg_adj_params &p, const F4 &X, const F4 &star, const F4 &out,
-               const WG &sa, const WG &sb, bool need_out = true) {
+               const WG *sa = nullptr, const WG *sb = nullptr, bool need_out = true) {
     if (p.precision == ZG_MIXED) heun_step_t<float>(a, st, p, X, star, out, sa, sb, need_out);
     else heun_step_t<double>(a, st, p, X, star, out, sa, sb, need_out);
 }
-WG scratch(const zg_adj *a) { return WG{a->W, a->gx, a->gy}; }
 WG seg_stage(const zg_adj *a, int b, int t, int stage) {
     return WG{a->segW[b][2 * t + stage], a->segGx[b][2 * t + stage], a->segGy[b][2 * t + stage]};
 }
@@ -676,9 +689,10 @@ WG seg_stage(const zg_adj *a, int b, int t, int stage) {
 void recompute(zg_adj *a, cudaStream_t st, const zg_adj_params &p, int sg, int len) {
     const int b = sg & 1;
     copy4(a, st, a->seg[b][0], a->ckpt[sg]);
-    for (int t = 0; t < len; ++t)
-        heun_step(a, st, p, a->seg[b][t], a->segstar[b][t], a->seg[b][t + 1], seg_stage(a, b, t, 0),
-                  seg_stage(a, b, t, 1), t + 1 < len);
+    for (int t = 0; t < len; ++t) {
+        const WG sa = seg_stage(a, b, t, 0), sb = seg_stage(a, b, t, 1);
+        heun_step(a, st, p, a->seg[b][t], a->segstar[b][t], a->seg[b][t + 1], &sa, &sb, t + 1 < len);
+    }
 }
 
 // out = base_coef * base + add + L'(X)^T (coef * mu), with X's primitive
@@ -765,6 +779,8 @@ int zg_adj_create(zg_adj **out, int device, int nx, int ny, double x_min, double
     a->g.hx = (x_max - x_min) / nx;
     a->g.hy = (y_max - y_min) / ny;
     a->g.vol = a->g.hx * a->g.hy;
+    a->g.i2x = 0.5 / a->g.hx;
+    a->g.i2y = 0.5 / a->g.hy;
     a->g.x0 = x_min;
     a->g.y0 = y_min;
     DevGuard gd(device);
@@ -833,7 +849,7 @@ int zg_adj_forward(zg_adj *a, const zg_adj_params *p, const double *rho, const d
     ++a->launches;
     F4 cur = a->Ua, nxt = a->Ub;
     for (int s = 0; s < p->steps; ++s) {
-        heun_step(a, a->stream, *p, cur, a->Ustar, nxt, scratch(a), scratch(a));
+        heun_step(a, a->stream, *p, cur, a->Ustar, nxt);
         std::swap(cur, nxt);
     }
     cudaMemsetAsync(a->d_acc, 0, 2 * nacc(a) * sizeof(double), a->stream);
@@ -878,14 +894,14 @@ int zg_adj_gradient(zg_adj *a, const zg_adj_params *p, const double *rho, const 
         if (s >= keep0) {
             const int sg = s / K, t = s - sg * K, b = sg & 1;
             if (t == 0) copy4(a, a->stream, a->seg[b][0], cur);
-            heun_step(a, a->stream, *p, a->seg[b][t], a->segstar[b][t], a->seg[b][t + 1], seg_stage(a, b, t, 0),
-                      seg_stage(a, b, t, 1));
+            const WG sa = seg_stage(a, b, t, 0), sb = seg_stage(a, b, t, 1);
+            heun_step(a, a->stream, *p, a->seg[b][t], a->segstar[b][t], a->seg[b][t + 1], &sa, &sb);
             cur = a->seg[b][t + 1];
             continue;
         }
         bool keep = (s + 1) % K == 0 && (s + 1) / K < nseg;
         F4 nxt = keep ? a->ckpt[(s + 1) / K] : (cur.f[0] == a->Ua.f[0] ? a->Ub : a->Ua);
-        heun_step(a, a->stream, *p, cur, a->Ustar, nxt, scratch(a), scratch(a));
+        heun_step(a, a->stream, *p, cur, a->Ustar, nxt);
         cur = nxt;
     }
     // J and lambda^N
