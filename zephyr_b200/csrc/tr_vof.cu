@@ -741,6 +741,9 @@ __device__ __forceinline__ void append(int *count, int *list, bool want, int val
 
 // Every face of the update: CRP fluxes directly; VOF fluxes directly where
 // they clip no polygon, the rest onto the face work list.
+// PLAIN: the VOF method, which stores nothing here; without the other methods'
+// formulas the kernel needs half the registers (68 -> 32; 2048 x 1434: 35 -> 24 us).
+template <bool PLAIN>
 __global__ void __launch_bounds__(BLOCK) k_flux_classify(TrArgs a, int dir) {
     const long long t = (long long)blockIdx.x * BLOCK + threadIdx.x;
     const bool live = t < n_faces(a.m, dir);
@@ -749,10 +752,10 @@ __global__ void __launch_bounds__(BLOCK) k_flux_classify(TrArgs a, int dir) {
     Face f;
     if (live) {
         f = face_at(a.m, dir, t, is_x, slot);
-        defer = vof_type(a.method) && face_needs_polygon(a, f, dir);
+        defer = (PLAIN || vof_type(a.method)) && face_needs_polygon(a, f, dir);
         // plain VOF: a face that clips no polygon carries +-0, which the
         // update skips (k_update); nothing to store
-        if (!defer && a.method != VOF) {
+        if (!PLAIN && !defer) {
             double fa, fb;
             face_fluxes<false>(a, f, dir, fa, fb);
             store_face(a, is_x, slot, fa, fb);
@@ -799,7 +802,8 @@ __global__ void __launch_bounds__(BLOCK) k_update(TrArgs a, int dir) {
         if (j > 0 && carries_flux(a, y_face(a.m, i, j), dir)) fl += a.fyb[(size_t)i * (ny + 1) + j];
         if (j < ny - 1 && carries_flux(a, y_face(a.m, i, j + 1), dir)) fl += a.fya[(size_t)i * (ny + 1) + j + 1];
     }
-    const double u2 = a.u[ic] - fl / a.m.vol;
+    // (most cells carry no flux: fl / vol is then a zero, see div_z)
+    const double u2 = fl == 0.0 ? a.u[ic] : a.u[ic] - fl / a.m.vol;
     a.u_next[ic] = dmax(0.0, dmin(u2, 1.0));
 }
 
@@ -1243,7 +1247,8 @@ void launch_flux(const TrArgs &a, int dir, cudaStream_t st) {
     const long long nf = (dir != 2 ? (nx - 1) * ny : 0) + (dir != 1 ? nx * (ny - 1) : 0);
     if (nf == 0) return;
     cudaMemsetAsync(a.count + 0, 0, sizeof(int), st);
-    k_flux_classify<<<blocks(nf), BLOCK, 0, st>>>(a, dir);
+    if (a.method == VOF) k_flux_classify<true><<<blocks(nf), BLOCK, 0, st>>>(a, dir);
+    else k_flux_classify<false><<<blocks(nf), BLOCK, 0, st>>>(a, dir);
     if (vof_type(a.method)) k_flux_list<<<list_blocks(k_flux_list, nf), BLOCK, 0, st>>>(a, dir);
 }
 
