@@ -590,7 +590,8 @@ __global__ void __launch_bounds__(BLOCK) k_grad2(MmArgs a) {
         const double rx = ncx - pcx, ry = ncy - pcy;
         const double d = rx * g.nx + ry * g.ny;
         const double nxx = d * g.nx, nyy = d * g.ny;
-        const double w = 1.0 * g.area / cube_rn(sqrt(nxx * nxx + nyy * nyy));
+        // area / |dr . n|^3, from the axis' table
+        const double w = s == 0 ? a.ax.wl[c.i] : (s == 1 ? a.ax.wh[c.i] : (s == 2 ? a.ay.wl[c.j] : a.ay.wh[c.j]));
         const double wdx = w * nxx, wdy = w * nyy;
         A00 += wdx * rx;
         A01 += wdx * ry;
@@ -868,9 +869,12 @@ __device__ __forceinline__ bool interp_pure(const MixD<NM> &mx, MSt<NM> &z) {
 
 // With composite fluxes (CRP modes): cells all of whose face values come out
 // pure take calc_flux's plain-HLLC branch here, with the same operations as
-// face_term2; a cell with a mixed face value goes to the work list, whose
-// faces k_stage2_faces evaluates one per thread and k_crp_update sums in slot
-// order.  The lean kernel keeps the Newton closures and the composite Riemann
+// face_term2; a cell with a mixed face value is in the work list, whose faces
+// k_stage2_faces evaluates one per thread and k_crp_update sums in slot order.
+// The list is made first (k_classify2), so that the listed faces, few and each
+// a long chain (103 us of 283 at 451^2 with 8 % of the warps resident), run
+// beside the other cells instead of after them: 451^2 295 -> 260 us a step.
+// The lean kernel keeps the Newton closures and the composite Riemann
 // solver out of the common path (fewer registers, more resident warps).
 // (four resident blocks: 128 registers, measured 9 % faster than three)
 // R = double: the reference's arithmetic.  R = float: the mixed form -- the
@@ -887,6 +891,34 @@ __device__ __forceinline__ PureSt<float> pure_f(const MSt<NM> &z) {
     for (int i = 0; i < NM; ++i) o.b[i] = (float)z.b.f[i];
     o.idx = frac_index(z.b);
     return o;
+}
+// The fractions of cell o's value at the offset (dx, dy), as shifted and
+// interp_pure form them: one material only?
+__device__ __forceinline__ bool pure_value(const MmArgs &a, int o, double dx, double dy) {
+    Frac<NM> b;
+#pragma unroll
+    for (int i = 0; i < NM; ++i) b.f[i] = a.zhalf.b[i][o] + (a.gx[6 + i][o] * dx + a.gy[6 + i][o] * dy);
+    normalize(b);
+    return frac_index(b) >= 0;
+}
+__global__ void __launch_bounds__(BLOCK) k_classify2(MmArgs a) {
+    const int ic = blockIdx.x * BLOCK + threadIdx.x;
+    if (ic >= a.mesh.n) return;
+    StructAcc c(a.mesh, ic);
+    const double pcx = c.cx(), pcy = c.cy();
+    bool pure = true;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        if (skip_face(a.dir, s)) continue;
+        FaceG g = c.face(s);
+        pure = pure && pure_value(a, ic, g.fcx - pcx, g.fcy - pcy);
+        if (pure && !is_boundary(g.flag)) {
+            double ncx, ncy;
+            neib_center(c, g, s, pcx, pcy, ncx, ncy);
+            pure = pure_value(a, g.nb, g.fcx - ncx, g.fcy - ncy);
+        }
+    }
+    if (!pure) a.list_crp[atomicAdd(&a.counts[0], 1)] = ic;
 }
 template <typename R>
 __global__ void __launch_bounds__(BLOCK, 4) k_stage2_pure(MmArgs a) {
@@ -914,10 +946,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_stage2_pure(MmArgs a) {
         } else {
             zp = ghost(zm, g);
         }
-        if (!pure) {
-            a.list_crp[atomicAdd(&a.counts[0], 1)] = ic;
-            return;
-        }
+        if (!pure) return;  // listed by k_classify2
         to_local(g.nx, g.ny, zm.vx, zm.vy, zm.vx, zm.vy);
         to_local(g.nx, g.ny, zp.vx, zp.vy, zp.vx, zp.vy);
         const double S = g.area;
@@ -992,16 +1021,19 @@ void launch_closure(const MmArgs &a, void *stream) {
 void launch_grad2(const MmArgs &a, void *stream) { k_grad2<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a); }
 void launch_grad_a(const MmArgs &a, void *stream) { k_grad_a<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a); }
 void launch_stage1(const MmArgs &a, void *stream) { k_stage1<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a); }
-void launch_stage2(const MmArgs &a, void *stream) {
-    cudaStream_t st = (cudaStream_t)stream;
-    if (a.crp == CRP_NONE) {
-        k_stage2<<<blocks(a), BLOCK, 0, st>>>(a);
-        return;
-    }
-    if (a.fp32_flux) k_stage2_pure<float><<<blocks(a), BLOCK, 0, st>>>(a);
-    else k_stage2_pure<double><<<blocks(a), BLOCK, 0, st>>>(a);
-    k_stage2_faces<<<std::min<unsigned>(4 * blocks(a), LIST_BLOCKS), BLOCK, 0, st>>>(a);
-    k_crp_update<<<std::min<unsigned>(blocks(a), LIST_BLOCKS), BLOCK, 0, st>>>(a);
+void launch_stage2_all(const MmArgs &a, void *stream) { k_stage2<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a); }
+void launch_classify2(const MmArgs &a, void *stream) {
+    k_classify2<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a);
+}
+void launch_stage2_pure(const MmArgs &a, void *stream) {
+    if (a.fp32_flux) k_stage2_pure<float><<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a);
+    else k_stage2_pure<double><<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a);
+}
+void launch_stage2_faces(const MmArgs &a, void *stream) {
+    k_stage2_faces<<<std::min<unsigned>(4 * blocks(a), LIST_BLOCKS), BLOCK, 0, (cudaStream_t)stream>>>(a);
+}
+void launch_stage2_update(const MmArgs &a, void *stream) {
+    k_crp_update<<<std::min<unsigned>(blocks(a), LIST_BLOCKS), BLOCK, 0, (cudaStream_t)stream>>>(a);
 }
 void launch_flags(const MmArgs &a, int *flags, void *stream) {
     k_flags<<<blocks(a), BLOCK, 0, (cudaStream_t)stream>>>(a, flags);

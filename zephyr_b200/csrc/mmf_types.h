@@ -25,6 +25,7 @@ struct MmField {
 
 struct MmArgs {
     StructMesh mesh;
+    ptile::Axis ax, ay;  // per-axis least-squares weights (second-order gradients)
     MixD<NMAT> mix;
     int crp;
     int fp32_flux;  // mixed form: FP32 face arithmetic in the pure-stencil kernel
@@ -83,7 +84,13 @@ void launch_flags(const MmArgs &a, int *flags, void *stream);
 // second order: compute_grad, fluxes_stage1, fluxes_stage2 (mm_fluid.cpp:439-680)
 void launch_grad2(const MmArgs &a, void *stream);
 void launch_stage1(const MmArgs &a, void *stream);
-void launch_stage2(const MmArgs &a, void *stream);
+void launch_stage2_all(const MmArgs &a, void *stream);  // every face of every cell (CRP mode NONE)
+// CRP modes: the list of cells with a mixed face value, the other cells, the
+// listed cells' faces (these two may run side by side), the listed cells' sums
+void launch_classify2(const MmArgs &a, void *stream);
+void launch_stage2_pure(const MmArgs &a, void *stream);
+void launch_stage2_faces(const MmArgs &a, void *stream);
+void launch_stage2_update(const MmArgs &a, void *stream);
 void launch_make_states(const MmArgs &a, const double *rho, const double *vx, const double *vy, const double *P,
                         const double *beta, void *stream);
 // the n cell states as the 14 doubles per cell of zg_mmf_state_download, and

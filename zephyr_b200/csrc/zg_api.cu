@@ -53,12 +53,10 @@ struct zg_ctx {
     SlotMesh smesh{};
     void *d_slot = nullptr;    // slot-mesh arrays
     void *d_axial = nullptr;   // axisymmetric volume_alt / area_alt of a slot mesh
-    double *d_geo = nullptr;  // all geometry tables
-    double *d_tgeo = nullptr;  // per-axis tables of the tiled kernels, FP64 then FP32
+    double *d_geo = nullptr;  // all geometry tables of a rectangle, one allocation
     tiled::AxisGeo<double> ax64{}, ay64{};
     tiled::AxisGeo<float> ax32{}, ay32{};
-    double *d_pgeo = nullptr;  // per-axis tables of the PARITY tile kernels
-    ptile::Axis pax{}, pay{};
+    ptile::Axis pax{}, pay{};  // tables of the PARITY tile kernels
     int cap = 0;  // cells every per-cell field holds (n, or the adaptive mesh's capacity)
 
     // adaptive mesh (AmrCells layout on the device)
@@ -225,8 +223,6 @@ void free_solver(zg_ctx *c) {
 
 void free_mesh(zg_ctx *c) {
     cudaFree(c->d_geo);
-    cudaFree(c->d_tgeo);
-    cudaFree(c->d_pgeo);
     cudaFree(c->d_slot);
     cudaFree(c->d_axial);
     c->d_axial = nullptr;
@@ -240,8 +236,6 @@ void free_mesh(zg_ctx *c) {
     c->grad_ordered = false;
     if (c->state_mode == STATE_ORDERED_MIXED) c->state_mode = ZG_MIXED;
     c->d_geo = nullptr;
-    c->d_tgeo = nullptr;
-    c->d_pgeo = nullptr;
     c->d_slot = nullptr;
     c->d_amr = nullptr;
     c->d_amr_scratch = nullptr;
@@ -1050,7 +1044,6 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
         i2y[j] = 0.0 * 0.0 + d * d + 0.0 * 0.0;
     }
     size_t total = (size_t)(nx + 1) + (ny + 1) + 3 * (size_t)nx + 3 * (size_t)ny + 2 * (size_t)nx + 2 * (size_t)ny;
-    ZG_CUDA(c, cudaMalloc(&c->d_geo, total * sizeof(double)));
     std::vector<double> host;
     host.reserve(total);
     auto put = [&host](const std::vector<double> &v) {
@@ -1060,20 +1053,22 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
     };
     size_t oX = put(X), oY = put(Y), ocx = put(cx), ocy = put(cy), ofx = put(fxm), ofy = put(fym),
            oix = put(i2x), oiy = put(i2y);
-    ZG_CUDA(c, cudaMemcpy(c->d_geo, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
-
     // per-axis tables of the tiled kernels (FP64 and FP32 copies)
+    const std::vector<double> tx = axis_tables(X, cx, fxm, (y_max - y_min) / ny, bc[0], bc[1]);
+    const std::vector<double> ty = axis_tables(Y, cy, fym, (x_max - x_min) / nx, bc[2], bc[3]);
+    const size_t otx = put(tx), oty = put(ty);
+    // and of the PARITY tile kernels
+    double seam_x[2], seam_y[2];
+    const size_t opx = put(parity_tables(X, cx, fxm, (y_max - y_min) / ny, seam_x)),
+                 opy = put(parity_tables(Y, cy, fym, (x_max - x_min) / nx, seam_y));
+    const size_t nd = tx.size() + ty.size(), of32 = host.size();
+    host.resize(of32 + (nd + 1) / 2);
+    float *f32h = reinterpret_cast<float *>(host.data() + of32);
+    std::copy(tx.begin(), tx.end(), f32h);
+    std::copy(ty.begin(), ty.end(), f32h + tx.size());
+    ZG_CUDA(c, cudaMalloc(&c->d_geo, host.size() * sizeof(double)));
+    ZG_CUDA(c, cudaMemcpy(c->d_geo, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
     {
-        std::vector<double> tx = axis_tables(X, cx, fxm, (y_max - y_min) / ny, bc[0], bc[1]);
-        std::vector<double> ty = axis_tables(Y, cy, fym, (x_max - x_min) / nx, bc[2], bc[3]);
-        size_t nd = tx.size() + ty.size();
-        ZG_CUDA(c, cudaMalloc(&c->d_tgeo, nd * (sizeof(double) + sizeof(float))));
-        std::vector<double> all(tx);
-        all.insert(all.end(), ty.begin(), ty.end());
-        std::vector<float> allf(all.begin(), all.end());
-        ZG_CUDA(c, cudaMemcpy(c->d_tgeo, all.data(), nd * sizeof(double), cudaMemcpyHostToDevice));
-        float *f32 = reinterpret_cast<float *>(c->d_tgeo + nd);
-        ZG_CUDA(c, cudaMemcpy(f32, allf.data(), nd * sizeof(float), cudaMemcpyHostToDevice));
         auto fill = [](auto &g, auto *base, int n) {
             g.wl = base;
             g.wh = base + n;
@@ -1084,26 +1079,17 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
             g.oh = base + 6 * (size_t)n;
             g.om = base + 7 * (size_t)n;
         };
-        fill(c->ax64, c->d_tgeo, nx);
-        fill(c->ay64, c->d_tgeo + tx.size(), ny);
+        float *f32 = reinterpret_cast<float *>(c->d_geo + of32);
+        fill(c->ax64, c->d_geo + otx, nx);
+        fill(c->ay64, c->d_geo + oty, ny);
         fill(c->ax32, f32, nx);
         fill(c->ay32, f32 + tx.size(), ny);
-    }
-
-    // per-axis tables of the PARITY tile kernels
-    {
-        double sx[2], sy[2];
-        std::vector<double> t = parity_tables(X, cx, fxm, (y_max - y_min) / ny, sx);
-        const std::vector<double> ty = parity_tables(Y, cy, fym, (x_max - x_min) / nx, sy);
-        t.insert(t.end(), ty.begin(), ty.end());
-        ZG_CUDA(c, cudaMalloc(&c->d_pgeo, t.size() * sizeof(double)));
-        ZG_CUDA(c, cudaMemcpy(c->d_pgeo, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
         auto axis = [](const double *b, size_t n, const double seam[2]) {
             return ptile::Axis{b,         b + n,     b + 2 * n, b + 3 * n, b + 4 * n,
                                b + 5 * n, b + 6 * n, b + 7 * n, seam[0],   seam[1]};
         };
-        c->pax = axis(c->d_pgeo, (size_t)nx, sx);
-        c->pay = axis(c->d_pgeo + 8 * (size_t)nx, (size_t)ny, sy);
+        c->pax = axis(c->d_geo + opx, (size_t)nx, seam_x);
+        c->pay = axis(c->d_geo + opy, (size_t)ny, seam_y);
     }
 
     StructMesh &m = c->mesh;
@@ -1581,6 +1567,8 @@ double ideal_ref_density(double gamma, double Cv, double P, double T) {
 mmf::MmArgs make_mm_args(const zg_ctx *c) {
     mmf::MmArgs a{};
     a.mesh = c->mesh;
+    a.ax = c->pax;
+    a.ay = c->pay;
     for (int i = 0; i < mmf::NMAT; ++i) {
         const zg_material &m = c->mpar.materials[i];
         a.mix.mat[i] = {m.kind == ZG_EOS_STIFFENED ? 1 : 0, m.gamma, m.P0, m.e0, m.Cv, m.T0, m.rho_ref};
@@ -1671,12 +1659,31 @@ int enqueue_mm_step(zg_ctx *c) {
         a.dt_scale = scale;
         if (!first_order && sub++ > 0) cudaMemsetAsync(a.counts, 0, 2 * sizeof(int), c->stream);  // empty work lists
         if (c->mpar.accuracy == 2) {
-            // MmFluid::integrate, second order (mm_fluid.cpp:152-168)
+            // MmFluid::integrate, second order (mm_fluid.cpp:152-168).  The
+            // side stream carries the interface reconstruction beside the
+            // gradients and the half step, then the faces of the listed cells
+            // beside the other cells.
+            const bool crp = c->mpar.crp_mode != ZG_CRP_NONE;
+            if (c->mpar.crp_mode == ZG_CRP_PLIC) {
+                cudaEventRecord(c->ev_fork, c->stream);
+                cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+                timed_on(c, ZG_K_MM_RECOVER, c->side, [&] { mmf::launch_recover(a, (void *)c->side); });
+            }
             timed(c, ZG_K_MM_GRAD, [&] { mmf::launch_grad2(a, st); });
             if (c->mpar.crp_mode == ZG_CRP_MUSCL) timed(c, ZG_K_MM_GRAD, [&] { mmf::launch_grad_a(a, st); });
-            if (c->mpar.crp_mode == ZG_CRP_PLIC) timed(c, ZG_K_MM_RECOVER, [&] { mmf::launch_recover(a, st); });
             timed(c, ZG_K_MM_STAGE1, [&] { mmf::launch_stage1(a, st); });
-            timed(c, ZG_K_MM_STAGE2, [&] { mmf::launch_stage2(a, st); });
+            if (!crp) {
+                timed(c, ZG_K_MM_STAGE2, [&] { mmf::launch_stage2_all(a, st); });
+            } else {
+                timed(c, ZG_K_MM_STAGE2, [&] { mmf::launch_classify2(a, st); });
+                cudaEventRecord(c->ev_dt, c->stream);
+                cudaStreamWaitEvent(c->side, c->ev_dt, 0);
+                timed_on(c, ZG_K_MM_CRP, c->side, [&] { mmf::launch_stage2_faces(a, (void *)c->side); });
+                timed(c, ZG_K_MM_STAGE2, [&] { mmf::launch_stage2_pure(a, st); });
+                cudaEventRecord(c->ev_join, c->side);
+                cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+                timed(c, ZG_K_MM_STAGE2, [&] { mmf::launch_stage2_update(a, st); });
+            }
             std::swap(c->mz, c->mznext);
             return;
         }
@@ -2753,11 +2760,7 @@ int zg_amr_enable(zg_ctx *c, int max_level, int capacity) {
     ZG_CUDA(c, cudaStreamSynchronize(c->stream));
     // the rectangle's axis tables are not used on a slot mesh
     cudaFree(c->d_geo);
-    cudaFree(c->d_tgeo);
-    cudaFree(c->d_pgeo);
     c->d_geo = nullptr;
-    c->d_tgeo = nullptr;
-    c->d_pgeo = nullptr;
     c->ax64 = c->ay64 = tiled::AxisGeo<double>{};
     c->ax32 = c->ay32 = tiled::AxisGeo<float>{};
     c->cap = capacity;
