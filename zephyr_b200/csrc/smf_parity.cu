@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "smf_parity_tile.cuh"
+#include "smf_slot_parity.cuh"
 #include "smf_struct.cuh"
 
 namespace zg {
@@ -42,7 +43,7 @@ static void flux1_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream
 }
 template <int FX>
 static void stage2_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
-    if (slots) k_stage2<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
+    if (slots) slotpar::k_stage2_4<FX><<<slotpar::blocks(a), slotpar::BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
     else k_stage2<StructAcc, BLOCK, 1, -1><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
 }
 template <int FX>
@@ -67,8 +68,20 @@ static void heun_fx(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, dou
 void launch_flux1(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
     ZG_FLUX_FAMILY(flux1_fx, a, dt_next, slots, stream);
 }
-void launch_grad(const SmfArgs &a, PrimPtr z, bool slots, void *stream) { ZG_DISPATCH(k_grad, a, z); }
-void launch_stage1(const SmfArgs &a, bool slots, void *stream) { ZG_DISPATCH(k_stage1, a); }
+void launch_grad(const SmfArgs &a, PrimPtr z, bool slots, void *stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (slots) slotpar::k_grad4<false><<<slotpar::blocks(a), slotpar::BLOCK, 0, st>>>(a, z);
+    else k_grad<StructAcc, BLOCK><<<blocks(a, false), BLOCK, 0, st>>>(a, z);
+}
+void launch_grad_stage1(const SmfArgs &a, bool slots, void *stream) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (slots) {
+        slotpar::k_grad4<true><<<slotpar::blocks(a), slotpar::BLOCK, 0, st>>>(a, a.z);
+    } else {
+        k_grad<StructAcc, BLOCK><<<blocks(a, false), BLOCK, 0, st>>>(a, a.z);
+        k_stage1<StructAcc, BLOCK><<<blocks(a, false), BLOCK, 0, st>>>(a);
+    }
+}
 void launch_stage2(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
     ZG_FLUX_FAMILY(stage2_fx, a, dt_next, slots, stream);
 }

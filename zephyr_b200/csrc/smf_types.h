@@ -85,7 +85,8 @@ void launch_dt(const SmfArgs &a, PrimPtr z, bool slots, void *stream);
 // dt_next (the last kernel of a step): the next step's dt goes there
 void launch_flux1(const SmfArgs &a, double *dt_next, bool slots, void *stream);
 void launch_grad(const SmfArgs &a, PrimPtr z, bool slots, void *stream);
-void launch_stage1(const SmfArgs &a, bool slots, void *stream);
+// gradients of a.z and the predictor (one kernel on a slot mesh, two on a rectangle)
+void launch_grad_stage1(const SmfArgs &a, bool slots, void *stream);
 void launch_stage2(const SmfArgs &a, double *dt_next, bool slots, void *stream);
 void launch_heun(const SmfArgs &a, PrimPtr zin, PrimPtr zout, bool final, double *dt_next, bool slots, void *stream);
 void launch_flags(const SmfArgs &a, int *flags, bool slots, void *stream);

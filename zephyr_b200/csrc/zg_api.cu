@@ -602,8 +602,8 @@ int enqueue_parity_step(zg_ctx *c) {
         tile(ZG_K_HEUN_A, ptile::HEUN_A, c->z, c->zhalf);
         tile(ZG_K_HEUN_B, ptile::HEUN_B, c->zhalf, c->znext);
     } else if (pc) {
-        timed(c, ZG_K_GRAD, [&] { parity::launch_grad(a, c->z, c->slots, st); });
-        timed(c, ZG_K_STAGE1, [&] { parity::launch_stage1(a, c->slots, st); });
+        if (!c->slots) ++c->launches;
+        timed(c, ZG_K_STAGE1, [&] { parity::launch_grad_stage1(a, c->slots, st); });
         timed(c, ZG_K_STAGE2, [&] { parity::launch_stage2(a, next, c->slots, st); });
     } else {
         timed(c, ZG_K_GRAD, [&] { parity::launch_grad(a, c->z, c->slots, st); });
