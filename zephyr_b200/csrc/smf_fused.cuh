@@ -645,6 +645,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
 
 template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
 __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<R> f, StepConst<R> k) {
+    after_previous();
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
     if (i0 >= 2 && i0 + TH + 2 <= a.mesh.nx && j0 >= 2 && j0 + 32 <= a.mesh.ny)
         step_tile<R, MIXED, MODE, LIM, TH, true>(a, f, k);
@@ -667,7 +668,7 @@ inline void launch_fused_stage(const SmfArgs &a, const Fields<R> &f, cudaStream_
     }
     dim3 block(32, TH + 2);
     dim3 grid((a.mesh.ny + 29) / 30, (a.mesh.nx + TH - 1) / TH);
-    kern<<<grid, block, L::bytes, s>>>(a, f, step_const<R>(a));
+    launch_after(kern, grid, block, L::bytes, s, a, f, step_const<R>(a));
 }
 
 // One stage (FUSED_PC, FUSED_HEUN_A or FUSED_HEUN_B) with the limiter

@@ -39,7 +39,7 @@ void launch_dt(const SmfArgs &a, PrimPtr z, bool slots, void *stream) {
 template <int FX>
 static void flux1_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream) {
     if (slots) k_flux1<SlotAcc, BLOCK, 1, FX><<<blocks(a, true), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
-    else k_flux1<StructAcc, BLOCK, 1, FX><<<blocks(a, false), BLOCK, 0, (cudaStream_t)stream>>>(a, dt_next);
+    else launch_after(k_flux1<StructAcc, BLOCK, 1, FX>, blocks(a, false), BLOCK, 0, (cudaStream_t)stream, a, dt_next);
 }
 template <int FX>
 static void stage2_fx(const SmfArgs &a, double *dt_next, bool slots, void *stream) {

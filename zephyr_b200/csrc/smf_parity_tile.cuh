@@ -555,6 +555,7 @@ __device__ __forceinline__ void tile(const Args &A) {
 
 template <int MODE, int LIM, bool HLL, int TH, int MINB>
 __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_tile(const __grid_constant__ Args A) {
+    after_previous();
     constexpr int H = Layout<MODE, TH>::H;
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
     if (i0 >= H && i0 + TH + H <= A.a.mesh.nx && j0 >= H && j0 + 30 + H <= A.a.mesh.ny)
@@ -575,7 +576,7 @@ inline void launch(const Args &A, cudaStream_t s) {
         if (dev < 64) attr_set |= 1ull << dev;
     }
     const StructMesh &m = A.a.mesh;
-    kern<<<dim3((m.ny + 29) / 30, (m.nx + TH - 1) / TH), dim3(32, TH + 2), L::bytes, s>>>(A);
+    launch_after(kern, dim3((m.ny + 29) / 30, (m.nx + TH - 1) / TH), dim3(32, TH + 2), L::bytes, s, A);
 }
 
 }  // namespace ptile

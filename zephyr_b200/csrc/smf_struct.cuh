@@ -30,6 +30,7 @@ struct FaceG {
 
 // Uniform rectangle.
 struct StructAcc {
+    static constexpr bool SLOTS = false;
     static constexpr int NSLOT = 4;
     static constexpr bool UNIT_NORMALS = true;  // axis normals: no normalisation
     static constexpr bool LSM_TWO_PASS = false;
@@ -99,6 +100,7 @@ struct StructAcc {
 
 // Mesh given slot by slot (AMR).
 struct SlotAcc {
+    static constexpr bool SLOTS = true;
     static constexpr int NSLOT = 8;
     static constexpr bool UNIT_NORMALS = false;
     static constexpr bool LSM_TWO_PASS = false;
@@ -141,6 +143,7 @@ struct SlotAcc {
 // second half (subface_nodes2d).  Used by the FAST slot kernels; on dyadic
 // meshes it reproduces the stored geometry exactly.
 struct SlotFastAcc {
+    static constexpr bool SLOTS = true;
     static constexpr int NSLOT = 8;
     static constexpr bool UNIT_NORMALS = true;
     static constexpr bool LSM_TWO_PASS = true;
@@ -379,6 +382,7 @@ __device__ inline void update(Cons &q, double coef, const Cons &F) {
 // K2: first-order step (sm_fluid.cpp:127-174).
 template <class Acc, int BLOCK, int MINB = 1, int FX = -1>
 __global__ void __launch_bounds__(BLOCK, MINB) k_flux1(SmfArgs a, double *dt_next = nullptr) {
+    if (!Acc::SLOTS) after_previous();
     const int ic = blockIdx.x * BLOCK + threadIdx.x;
     unsigned long long best = 0x7FEFFFFFFFFFFFFFull;
     if (ic < Acc::n(a)) {

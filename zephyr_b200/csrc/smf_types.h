@@ -4,9 +4,40 @@
 
 #include <cstdint>
 
+#include <cuda_runtime.h>
+
 #include "smf_math.cuh"
 
 namespace zg {
+
+// Programmatic dependent launch of the rectangle's step kernels: a kernel may
+// be placed on the SMs once every block of the one before has started, and
+// waits in after_previous() until that one has finished and its writes are
+// visible.  Hides part of the launch latency between the steps of small meshes
+// (256^2 first order 12.4 -> 11.1 us a step, 129 x 67 second order 11.1 -> 10.1).
+// Not for the marching kernels, whose grids fill the GPU exactly once: Heun's
+// two stages want different shared-memory carve-outs, and a stage placed under
+// the other's got three blocks on an SM instead of four (2048^2 430 -> 547 us).
+#ifdef __CUDACC__
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+#endif
 
 // Structured rectangle, geometry in per-axis tables filled on the host with
 // the reference's formulas (amr_cells_gen.cpp:128-253).
