@@ -61,7 +61,7 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
     // HLLC and HLL get kernels without the other fluxes' code (registers)
     if (a.flux == FLUX_HLLC || a.flux == FLUX_HLL) {
         switch (mode) {
-            case 0: tiled::k_faces<double, false, 0, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
+            case 0: launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB, false>, grid, block, 0, s, a, f); break;
             case 1: tiled::k_faces<double, false, 1, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             case 2: tiled::k_faces<double, false, 2, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             default: tiled::k_faces<double, false, 3, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
@@ -69,7 +69,7 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
         return;
     }
     switch (mode) {
-        case 0: tiled::k_faces<double, false, 0, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
+        case 0: launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB>, grid, block, 0, s, a, f); break;
         case 1: tiled::k_faces<double, false, 1, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         case 2: tiled::k_faces<double, false, 2, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         default: tiled::k_faces<double, false, 3, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
@@ -99,7 +99,8 @@ void launch_step(const SmfArgs &a, const Fields<double> &f, int mode, void *stre
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_FAST_MARCH_MINB);
     constexpr int TH = ZG_FAST_FUSED_TH;
     const long long tiles = (long long)((a.mesh.ny + 29) / 30) * ((a.mesh.nx + TH - 1) / TH);
-    if (sp.rows >= (mode == tiled::FUSED_PC ? MARCH_MIN_ROWS_PC : MARCH_MIN_ROWS_HEUN))
+    if (tiled::march_limiter(a.limiter) &&
+        sp.rows >= (mode == tiled::FUSED_PC ? MARCH_MIN_ROWS_PC : MARCH_MIN_ROWS_HEUN))
         tiled::march_dispatch<double, false, ZG_FAST_MARCH_MINB>(a, f, mode, sp, s);
     else if (4 * tiles <= 3 * 148)
         tiled::fused_dispatch<double, false, 2, 4>(a, f, mode, s);

@@ -647,10 +647,14 @@ template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
 __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<R> f, StepConst<R> k) {
     after_previous();
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
-    if (i0 >= 2 && i0 + TH + 2 <= a.mesh.nx && j0 >= 2 && j0 + 32 <= a.mesh.ny)
-        step_tile<R, MIXED, MODE, LIM, TH, true>(a, f, k);
-    else
-        step_tile<R, MIXED, MODE, LIM, TH, false>(a, f, k);
+    // (a limiter chosen at run time: one copy of its code, see march_limiter)
+    if constexpr (LIM >= 0) {
+        if (i0 >= 2 && i0 + TH + 2 <= a.mesh.nx && j0 >= 2 && j0 + 32 <= a.mesh.ny) {
+            step_tile<R, MIXED, MODE, LIM, TH, true>(a, f, k);
+            return;
+        }
+    }
+    step_tile<R, MIXED, MODE, LIM, TH, false>(a, f, k);
 }
 
 // Launch one stage of the fused step on `stream` (dynamic shared memory of
@@ -680,6 +684,7 @@ inline void fused_stage(const SmfArgs &a, const Fields<R> &f, cudaStream_t s) {
         case LIM_VANALBADA1: launch_fused_stage<R, MIXED, MODE, LIM_VANALBADA1, TH, MINB>(a, f, s); break;
         case LIM_MC: launch_fused_stage<R, MIXED, MODE, LIM_MC, TH, MINB>(a, f, s); break;
         case LIM_MINMOD: launch_fused_stage<R, MIXED, MODE, LIM_MINMOD, TH, MINB>(a, f, s); break;
+        case LIM_VANLEER: launch_fused_stage<R, MIXED, MODE, LIM_VANLEER, TH, MINB>(a, f, s); break;
         default: launch_fused_stage<R, MIXED, MODE, -1, TH, MINB>(a, f, s); break;
     }
 }

@@ -582,8 +582,15 @@ inline void march_stage(const SmfArgs &a, const Fields<R> &f, const MarchSplit &
         case LIM_VANALBADA1: launch_march<R, MIXED, MODE, LIM_VANALBADA1, MINB>(a, f, sp, s); break;
         case LIM_MC: launch_march<R, MIXED, MODE, LIM_MC, MINB>(a, f, sp, s); break;
         case LIM_MINMOD: launch_march<R, MIXED, MODE, LIM_MINMOD, MINB>(a, f, sp, s); break;
-        default: launch_march<R, MIXED, MODE, -1, MINB>(a, f, sp, s); break;
+        default: launch_march<R, MIXED, MODE, LIM_VANLEER, MINB>(a, f, sp, s); break;
     }
+}
+// The limiters compiled into the march.  The others are chosen at run time, a
+// switch of thirteen forms in each of eight slopes, whose code (the tile
+// kernel's too: its INTERIOR copy is left out for them) outgrows the
+// instruction cache: van Leer through it 253 against 223 us at 1400^2.
+inline bool march_limiter(int lim) {
+    return lim == LIM_VANALBADA1 || lim == LIM_MC || lim == LIM_MINMOD || lim == LIM_VANLEER;
 }
 template <typename R, bool MIXED, int MINB>
 inline void march_dispatch(const SmfArgs &a, const Fields<R> &f, int mode, const MarchSplit &sp, cudaStream_t s) {

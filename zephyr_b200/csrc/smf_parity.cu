@@ -107,6 +107,7 @@ static void tile_lim(const ptile::Args &A, cudaStream_t s) {
         case LIM_VANALBADA1: tile_flux<MODE, LIM_VANALBADA1>(A, s); break;
         case LIM_MC: tile_flux<MODE, LIM_MC>(A, s); break;
         case LIM_MINMOD: tile_flux<MODE, LIM_MINMOD>(A, s); break;
+        case LIM_VANLEER: tile_flux<MODE, LIM_VANLEER>(A, s); break;
         default: tile_flux<MODE, -1>(A, s); break;
     }
 }

@@ -558,10 +558,14 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_tile(const __grid_const
     after_previous();
     constexpr int H = Layout<MODE, TH>::H;
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
-    if (i0 >= H && i0 + TH + H <= A.a.mesh.nx && j0 >= H && j0 + 30 + H <= A.a.mesh.ny)
-        tile<MODE, LIM, HLL, TH, true>(A);
-    else
-        tile<MODE, LIM, HLL, TH, false>(A);
+    // (a limiter chosen at run time: one copy of its code)
+    if constexpr (LIM >= 0) {
+        if (i0 >= H && i0 + TH + H <= A.a.mesh.nx && j0 >= H && j0 + 30 + H <= A.a.mesh.ny) {
+            tile<MODE, LIM, HLL, TH, true>(A);
+            return;
+        }
+    }
+    tile<MODE, LIM, HLL, TH, false>(A);
 }
 
 template <int MODE, int LIM, bool HLL, int TH, int MINB>
