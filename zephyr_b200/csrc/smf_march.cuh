@@ -1,7 +1,7 @@
 // smf_march.cuh -- the second-order step of a structured rectangle with every
-// warp marching down the rows of its own strip of columns: the arithmetic of the fused tile kernel (smf_fused.cuh: limited
-// gradients, half step, face-once corrector, update, the next step's CFL
-// minimum) without block barriers.
+// warp marching down the rows of its own strip of columns: the arithmetic of
+// the fused tile kernel (smf_fused.cuh: limited gradients, half step, face-once
+// corrector, update, the next step's CFL minimum) without block barriers.
 //
 // A warp owns 28 columns: lane l holds column j0 - 2 + l, lanes 2..29 are
 // updated, the outer two on each side are the stencil's halo.  It walks the
@@ -21,8 +21,8 @@
 // they look: an atomic minimum per cell on the one CFL slot (190 us at 1024^2
 // against 88 with one per warp), and bad-value fallbacks as selects instead of
 // branches under a warp vote (317 against 301 us at 2048^2).
-// Measured (B200, one step, FP64 / MIXED): 2048^2 predictor-corrector 351 ->
-// 301 / 294 -> 250 us, Heun 541 -> 430 / 470 -> 321 us.
+// Measured (B200, one step, FP64 / MIXED): 2048^2 predictor-corrector 354 ->
+// 314 / 294 -> 250 us, Heun 541 -> 430 / 470 -> 321 us.
 #pragma once
 
 #include "smf_fused.cuh"
@@ -247,93 +247,6 @@ __device__ __forceinline__ void store_cell(const SmfArgs &a, const Fields<R> &f,
     cfl.add(a, i, j, zn, ri, live);
 }
 
-// ---- segments with an isolated cell (rare): every cell by itself ------------
-// Half-step state and slopes of cell ic = (i, j), from memory.
-template <typename R>
-struct CellHalf {
-    FS<R> h;
-    R g[2][4];
-    bool waiting;
-};
-template <typename R, bool MIXED, int LIM>
-__device__ __noinline__ void cell_half(const SmfArgs &a, const Fields<R> &f, const StepConst<R> &k, int i, int j,
-                                       double coef, CellHalf<R> &o) {
-    const StructMesh &m = a.mesh;
-    const EosR<R> eos = eos_as<R>(a.eos);
-    const int ic = i * m.ny + j;
-    const P5<R> z = ld5(f.w, ic);
-    o.h = FS<R>{z.r, z.u, z.v, z.p, z.e, R(0)};
-    o.waiting = f.wait_in[ic] > 0;
-    for (int q = 0; q < 4; ++q) {
-        const R own = f.w[q][ic];
-        R d[4];
-        for (int s = 0; s < 4; ++s) {
-            int flag;
-            const int nb = slot_nb(m, i, j, ic, s, flag);
-            const bool mirror = flag == BC_WALL && q == (s < 2 ? 1 : 2);
-            d[s] = (is_boundary(flag) ? (mirror ? -own : own) : f.w[q][nb]) - own;
-        }
-        o.g[0][q] = slope<LIM, R>(a.limiter, d[0], d[1], k.inv2hx, k.invhx);
-        o.g[1][q] = slope<LIM, R>(a.limiter, d[2], d[3], k.inv2hy, k.invhy);
-    }
-    const FS<R> h = half_step<R>(o.h, q_of<R, MIXED>(f, ic), o.g[0], o.g[1], k, eos, a.eos, m.hx, m.hy, coef);
-    if (!o.waiting) o.h = h;
-}
-// All lanes of the warp call it, with any cell of the mesh; `live` lanes
-// update theirs.
-template <typename R, bool MIXED, int LIM, bool HLL>
-__device__ __noinline__ void isolated_cell(const SmfArgs &a, const Fields<R> &f, const StepConst<R> &k, int i, int j,
-                                           bool live, double coef, WarpCfl &cfl) {
-    const StructMesh &m = a.mesh;
-    const EosR<R> eos = eos_as<R>(a.eos);
-    const int ic = i * m.ny + j;
-    CellHalf<R> own, other;
-    cell_half<R, MIXED, LIM>(a, f, k, i, j, coef, own);
-    double F[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int s = 0; s < 4; ++s) {
-        int flag;
-        const int nb = slot_nb(m, i, j, ic, s, flag);
-        const bool bnd = is_boundary(flag), high = (s & 1) != 0;
-        const int ax = s >> 1, in = nb / m.ny;
-        cell_half<R, MIXED, LIM>(a, f, k, in, nb - in * m.ny, coef, other);
-        const bool robust = own.waiting || other.waiting;  // (the cell itself on a boundary)
-        const R off = ax == 0 ? k.halfx : k.halfy;
-        FS<R> z = face_value<R>(own.h, own.g[ax], high ? off : -off, eos, k.igm1);
-        FS<R> zo = face_value<R>(other.h, other.g[ax], high ? -off : off, eos, k.igm1);
-        if (robust) {
-            z = own.h;
-            z.ri = rcp_r(z.r);
-            zo = other.h;
-            zo.ri = rcp_r(zo.r);
-        }
-        if (bnd) {
-            zo = z;
-            if (flag == BC_WALL) {
-                if (ax == 0) zo.u = -zo.u;
-                else zo.v = -zo.v;
-            }
-        }
-        FS<R> L = high ? z : zo, Rs = high ? zo : z;
-        if (ax == 1) {
-            L = FS<R>{L.r, L.v, L.u, L.p, L.e, L.ri};
-            Rs = FS<R>{Rs.r, Rs.v, Rs.u, Rs.p, Rs.e, Rs.ri};
-        }
-        C4<R> lf = march_flux<HLL, R>(L, Rs, eos);
-        if (robust) lf = hll_fs(L, Rs, eos);
-        const double w = (high ? 1.0 : -1.0) * (ax == 0 ? m.hy : m.hx);
-        F[0] += (double)lf.r * w;
-        F[1] += (double)(ax == 0 ? lf.mu : lf.mv) * w;
-        F[2] += (double)(ax == 0 ? lf.mv : lf.mu) * w;
-        F[3] += (double)lf.E * w;
-    }
-    C4<double> q = q_of<R, MIXED>(f, ic);
-    q.r -= coef * F[0];
-    q.mu -= coef * F[1];
-    q.mv -= coef * F[2];
-    q.E -= coef * F[3];
-    store_cell<R, MIXED, FUSED_PC>(a, f, i, j, live, q, f.wait_in[ic], cfl);
-}
-
 // One asynchronous copy of a lane's value (4 or 8 bytes) into shared memory.
 template <typename T>
 __device__ __forceinline__ void async_copy(T *dst, const T *src) {
@@ -388,15 +301,11 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
     auto row = [&](int i) { return (m.xper ? wrap_any(i, m.nx) : min(max(i, 0), m.nx - 1)) * m.ny + jc; };
     const double coef = dt / m.vol, hx = m.hx, hy = m.hy;
     WarpCfl cfl;
+    bool iso = false;  // an isolated cell in the segment or beside it
     if (PC) {
-        int waits = 0;
-        for (int g = i_lo - 1; g <= i_hi; ++g) waits |= f.wait_in[row(g)];  // counters are never negative
-        if (__any_sync(ALL, waits != 0)) {
-            for (int i = i_lo; i < i_hi; ++i)
-                isolated_cell<R, MIXED, LIM, HLL>(a, f, k, i, jc, live, coef, cfl);
-            cfl.commit(f.slot_nxt);
-            return;
-        }
+        int any = 0;
+        for (int g = i_lo - 1; g <= i_hi; ++g) any |= f.wait_in[row(g)];  // counters are never negative
+        iso = __any_sync(ALL, any != 0);
     }
     const EosR<R> eos = eos_as<R>(a.eos);
     // source of the stage: the state at t^n, or the Heun stage value z*
@@ -441,6 +350,14 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
     fetch_b(i_lo - 1, bc);
     async_commit();
     const int lu = max(l - 1, 0), ld = min(l + 1, 31);
+    // Isolated cells (sm_fluid.cpp:285-351) take no half step, and HLL runs
+    // between the cells' own states at their faces: branches of the one loop on
+    // a flag of the segment.  A second copy of the loop for such segments saves
+    // 0.6 % without them (312.5 against 314.4 us at 2048^2), but where both
+    // kinds run beside each other they do not fit the instruction cache (1 cell
+    // of 10^4 isolated: 380 us against 322; the tile kernel 355).
+    int wm = 0, wc = 0;  // counters of rows g - 1 and g
+    if (iso) wc = f.wait_in[row(i_lo - 1)];
 #pragma unroll 1
     for (int g = i_lo - 1; g <= i_hi; ++g) {
         async_wait();
@@ -472,12 +389,27 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
             gy[q] = slope<LIM, R>(a.limiter, nB - c, nT - c, k.inv2hy, k.invhy);
         }
         // ---- state the faces are reconstructed from: the half step, or z --
-        if (PC) h = half_step<R>(h, base(sc, bc), gx, gy, k, eos, a.eos, hx, hy, coef);
+        if (PC) {
+            const FS<R> hs = half_step<R>(h, base(sc, bc), gx, gy, k, eos, a.eos, hx, hy, coef);
+            if (!iso || wc == 0) h = hs;
+        }
+        FS<R> own = h;  // for an isolated cell's faces
+        int wp = 0;     // counter of row g + 1
+        if (iso) {
+            own.ri = rcp_r(h.r);
+            if (g < i_hi) wp = f.wait_in[row(g + 1)];
+        }
         // ---- faces between lanes l and l + 1 (frame of the +y normal) ------
         C4<R> fy;
         {
             FS<R> L = face_value<R>(h, gy, k.halfy, eos, k.igm1);
             FS<R> Rs = shfl_down_fs(face_value<R>(h, gy, -k.halfy, eos, k.igm1));
+            bool robust = false;
+            if (iso) {
+                const FS<R> next = shfl_down_fs(own);
+                robust = (wc | __shfl_down_sync(ALL, wc, 1)) != 0;
+                if (robust) L = own, Rs = next;
+            }
             if (sides) {  // past a side the mirror of the face's own state
                 if (j == -1) {
                     L = Rs;
@@ -489,13 +421,16 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 }
             }
             const FS<R> Ln{L.r, L.v, L.u, L.p, L.e, L.ri}, Rn{Rs.r, Rs.v, Rs.u, Rs.p, Rs.e, Rs.ri};
-            const C4<R> t = march_flux<HLL, R>(Ln, Rn, eos);
+            C4<R> t = march_flux<HLL, R>(Ln, Rn, eos);
+            if (!HLL && robust) t = hll_fs(Ln, Rn, eos);
             fy = C4<R>{t.r, t.mv, t.mu, t.E};
         }
         // ---- faces between rows g - 1 and g -------------------------------
         C4<R> fx{};
         if (g > i_lo - 1) {
             FS<R> L = up, Rs = face_value<R>(h, gx, -k.halfx, eos, k.igm1);
+            const bool robust = iso && (wm | wc) != 0;
+            if (robust) Rs = own;
             if (low) {
                 L = Rs;
                 if (m.bc[0] == BC_WALL) L.u = -L.u;
@@ -505,6 +440,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 if (m.bc[1] == BC_WALL) Rs.u = -Rs.u;
             }
             fx = march_flux<HLL, R>(L, Rs, eos);
+            if (!HLL && robust) fx = hll_fs(L, Rs, eos);
         }
         // ---- update of row g - 1 -------------------------------------------
         if (g > i_lo) {
@@ -524,7 +460,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 q.mv = 0.5 * (qn.mv + q.mv);
                 q.E = 0.5 * (qn.E + q.E);
             }
-            store_cell<R, MIXED, MODE>(a, f, g - 1, j, live, q, 0, cfl);
+            store_cell<R, MIXED, MODE>(a, f, g - 1, j, live, q, wm, cfl);
         }
         // ---- carry row g over -----------------------------------------------
         const C4<R> fb{__shfl_up_sync(ALL, fy.r, 1), __shfl_up_sync(ALL, fy.mu, 1), __shfl_up_sync(ALL, fy.mv, 1),
@@ -534,6 +470,9 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
         acc[2] = (-(double)fx.mv * hy - (double)fb.mv * hx) + (double)fy.mv * hx;
         acc[3] = (-(double)fx.E * hy - (double)fb.E * hx) + (double)fy.E * hx;
         up = face_value<R>(h, gx, k.halfx, eos, k.igm1);
+        if (iso && (wc | wp) != 0) up = own;
+        wm = wc;
+        wc = wp;
         const int t = sm;
         sm = sc;
         sc = sp;
@@ -588,7 +527,8 @@ inline void march_stage(const SmfArgs &a, const Fields<R> &f, const MarchSplit &
 // The limiters compiled into the march.  The others are chosen at run time, a
 // switch of thirteen forms in each of eight slopes, whose code (the tile
 // kernel's too: its INTERIOR copy is left out for them) outgrows the
-// instruction cache: van Leer through it 253 against 223 us at 1400^2.
+// instruction cache: van Leer through it 223 us at 1400^2 in the tile kernel,
+// compiled in 162.
 inline bool march_limiter(int lim) {
     return lim == LIM_VANALBADA1 || lim == LIM_MC || lim == LIM_MINMOD || lim == LIM_VANLEER;
 }

@@ -586,7 +586,12 @@ bool parity_tiles(const zg_ctx *c) {
 int enqueue_parity_step(zg_ctx *c) {
     if (c->par.accuracy == 2) c->grad_ordered = false;  // this step's gradients, in the mesh's order
     void *st = (void *)c->stream;
-    const bool have_dt = c->dt_next_ready, pc = c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR;
+    // A recorded step runs again on states it does not know: it brings its own
+    // dt pass, and leaves no minimum that a later step could take as computed.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(c->stream, &cs);
+    const bool live = cs == cudaStreamCaptureStatusNone;
+    const bool have_dt = c->dt_next_ready && live, pc = c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR;
     if (have_dt) std::swap(c->d_dt, c->d_dt2);
     SmfArgs a = make_args(c);
     if (!have_dt) timed(c, ZG_K_DT, [&] { parity::launch_dt(a, c->z, c->slots, st); });
@@ -615,7 +620,7 @@ int enqueue_parity_step(zg_ctx *c) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "kernel launch");
     std::swap(c->z, c->znext);  // Storage::swap of init and next (sm_fluid.cpp:368-370)
-    c->dt_next_ready = true;
+    c->dt_next_ready = live;
     c->cfl_valid = false;
     c->stepped = true;
     return ZG_OK;
