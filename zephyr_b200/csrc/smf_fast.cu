@@ -61,7 +61,10 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
     // HLLC and HLL get kernels without the other fluxes' code (registers)
     if (a.flux == FLUX_HLLC || a.flux == FLUX_HLL) {
         switch (mode) {
-            case 0: launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB, false>, grid, block, 0, s, a, f); break;
+            case 0:
+                if (early_first_order(grid)) launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB, false>, grid, block, 0, s, a, f);
+                else tiled::k_faces<double, false, 0, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f);
+                break;
             case 1: tiled::k_faces<double, false, 1, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             case 2: tiled::k_faces<double, false, 2, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             default: tiled::k_faces<double, false, 3, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
@@ -69,7 +72,10 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
         return;
     }
     switch (mode) {
-        case 0: launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB>, grid, block, 0, s, a, f); break;
+        case 0:
+                if (early_first_order(grid)) launch_after(tiled::k_faces<double, false, 0, TX, TY, FMINB>, grid, block, 0, s, a, f);
+                else tiled::k_faces<double, false, 0, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f);
+                break;
         case 1: tiled::k_faces<double, false, 1, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         case 2: tiled::k_faces<double, false, 2, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         default: tiled::k_faces<double, false, 3, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
@@ -88,7 +94,7 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
 #define ZG_FAST_MARCH_MINB 4
 #endif
 // The form by size, measured on B200 (us per step, march / tile):
-//   predictor-corrector  2048^2 301 / 332, 1200^2 111 / 122, 1024^2 85 / 89, 896^2 71 / 66
+//   predictor-corrector  2048^2 314 / 332, 1200^2 111 / 122, 1024^2 85 / 89, 896^2 71 / 66
 //   Heun                 2048^2 430 / 479, 1200^2 162 / 175, 1024^2 125 / 134, 896^2 104 / 101
 // so the march from 16 rows per segment on (1024^2).  Below, the tile kernel;
 // where its grid would leave a quarter of the SMs without a block, tiles of 2

@@ -515,28 +515,17 @@ inline void launch_march(const SmfArgs &a, const Fields<R> &f, const MarchSplit 
     else
         k_march<R, MIXED, MODE, LIM, false, MINB><<<blocks, nt, 0, s>>>(a, f, step_const<R>(a), sp.strips, sp.rows);
 }
-template <typename R, bool MIXED, int MINB, int MODE>
-inline void march_stage(const SmfArgs &a, const Fields<R> &f, const MarchSplit &sp, cudaStream_t s) {
-    switch (a.limiter) {
-        case LIM_VANALBADA1: launch_march<R, MIXED, MODE, LIM_VANALBADA1, MINB>(a, f, sp, s); break;
-        case LIM_MC: launch_march<R, MIXED, MODE, LIM_MC, MINB>(a, f, sp, s); break;
-        case LIM_MINMOD: launch_march<R, MIXED, MODE, LIM_MINMOD, MINB>(a, f, sp, s); break;
-        default: launch_march<R, MIXED, MODE, LIM_VANLEER, MINB>(a, f, sp, s); break;
-    }
-}
-// The limiters compiled into the march.  The others are chosen at run time, a
-// switch of thirteen forms in each of eight slopes, whose code (the tile
-// kernel's too: its INTERIOR copy is left out for them) outgrows the
-// instruction cache: van Leer through it 223 us at 1400^2 in the tile kernel,
-// compiled in 162.
-inline bool march_limiter(int lim) {
-    return lim == LIM_VANALBADA1 || lim == LIM_MC || lim == LIM_MINMOD || lim == LIM_VANLEER;
-}
+// The march runs van Albada 1, whose slope has a closed form.  The limiters that
+// are formed from the general refit keep more values alive, and 128 registers a
+// thread leave too few warps to cover their divisions: tile against march, FP64
+// at 2000^2 on smooth data: MC 402 / 461, minmod 365 / 395, van Leer 368 / 399 us
+// (van Albada 1: 338 / 314 at 2048^2); MIXED at 2048^2 MC 291 / 318.
+inline bool march_limiter(int lim) { return lim == LIM_VANALBADA1; }
 template <typename R, bool MIXED, int MINB>
 inline void march_dispatch(const SmfArgs &a, const Fields<R> &f, int mode, const MarchSplit &sp, cudaStream_t s) {
-    if (mode == FUSED_PC) march_stage<R, MIXED, MINB, FUSED_PC>(a, f, sp, s);
-    else if (mode == FUSED_HEUN_A) march_stage<R, MIXED, MINB, FUSED_HEUN_A>(a, f, sp, s);
-    else march_stage<R, MIXED, MINB, FUSED_HEUN_B>(a, f, sp, s);
+    if (mode == FUSED_PC) launch_march<R, MIXED, FUSED_PC, LIM_VANALBADA1, MINB>(a, f, sp, s);
+    else if (mode == FUSED_HEUN_A) launch_march<R, MIXED, FUSED_HEUN_A, LIM_VANALBADA1, MINB>(a, f, sp, s);
+    else launch_march<R, MIXED, FUSED_HEUN_B, LIM_VANALBADA1, MINB>(a, f, sp, s);
 }
 
 }  // namespace tiled

@@ -63,7 +63,10 @@ void launch_faces(const SmfArgs &a, const Fields<float> &f, int mode, void *stre
     // HLLC and HLL get kernels without the other fluxes' code (registers)
     if (a.flux == FLUX_HLLC || a.flux == FLUX_HLL) {
         switch (mode) {
-            case 0: launch_after(tiled::k_faces<float, true, 0, TX, TY, FMINB, false>, grid, block, 0, s, a, f); break;
+            case 0:
+                if (early_first_order(grid)) launch_after(tiled::k_faces<float, true, 0, TX, TY, FMINB, false>, grid, block, 0, s, a, f);
+                else tiled::k_faces<float, true, 0, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f);
+                break;
             case 1: tiled::k_faces<float, true, 1, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             case 2: tiled::k_faces<float, true, 2, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
             default: tiled::k_faces<float, true, 3, TX, TY, FMINB, false><<<grid, block, 0, s>>>(a, f); break;
@@ -71,7 +74,10 @@ void launch_faces(const SmfArgs &a, const Fields<float> &f, int mode, void *stre
         return;
     }
     switch (mode) {
-        case 0: launch_after(tiled::k_faces<float, true, 0, TX, TY, FMINB>, grid, block, 0, s, a, f); break;
+        case 0:
+                if (early_first_order(grid)) launch_after(tiled::k_faces<float, true, 0, TX, TY, FMINB>, grid, block, 0, s, a, f);
+                else tiled::k_faces<float, true, 0, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f);
+                break;
         case 1: tiled::k_faces<float, true, 1, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         case 2: tiled::k_faces<float, true, 2, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;
         default: tiled::k_faces<float, true, 3, TX, TY, FMINB><<<grid, block, 0, s>>>(a, f); break;

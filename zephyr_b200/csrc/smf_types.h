@@ -37,6 +37,15 @@ inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
+// k_faces' first-order step: early where both steps' blocks find SMs of their
+// own, or each fills the GPU twice over; in between the waiting blocks cost more
+// than the launch saves (us a step with / without, HLL: 100^2 4.9 / 6.2, 128^2
+// 7.2 / 6.2, 160^2 7.5 / 6.2, 256^2 7.9 / 8.2, 700^2 25.1 / 26.7; HLLC: 200^2 8.8 /
+// 8.2, 256^2 9.3 / 10.3).
+inline bool early_first_order(dim3 grid) {
+    const long long blocks = (long long)grid.x * grid.y;
+    return 2 * blocks <= 148 || blocks >= 2 * 148;
+}
 #endif
 
 // Structured rectangle, geometry in per-axis tables filled on the host with
