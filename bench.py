@@ -1051,7 +1051,7 @@ def run_ours(args, rank, world, local_rank):
         "warmup": args.warmup, "ms_per_step": ms / K, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": dict(config_of(args, w, cfg, world),
-                       form="FP64 (FAST kernels: one fused kernel per step, face-once tiles in shared memory)",
+                       form="FP64 (FAST kernels: one fused kernel per step, every face once)",
                        timing="headline timed without per-kernel events; the kernel split from a second run"),
         "roofline": roof, "kernels": kernels,
         "gpu_launches": int(launches + sum(v["launches"] for v in variants.values()) +

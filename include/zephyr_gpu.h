@@ -90,14 +90,16 @@ enum zg_scheme { ZG_SCHEME_PREDICTOR_CORRECTOR = 0, ZG_SCHEME_HEUN = 1 };
 /* Arithmetic of the face loop.  FP64 is the drop-in form. */
 enum zg_precision { ZG_FP64 = 0, ZG_MIXED = 1 };
 
-/* Kernel family.  PARITY evaluates every face flux from both sides in the
+/* Kernel family.  PARITY forms every face flux as both sides see it, in the
  * reference's order of operations without fused multiply-adds (bit-exact with
- * the reference); FAST computes each face once and lets the compiler fuse.
+ * the reference; second order with HLLC or HLL on a rectangle evaluates a
+ * face once and forms both views of it); FAST computes each face once and
+ * lets the compiler fuse.
  * On a rectangle, FAST runs each second-order stage with HLLC or HLL as ONE
- * kernel (gradients, predictor, faces and update of a tile in shared
- * memory); FAST_TWO_PASS keeps the earlier two kernels per stage (gradients
- * and predictor stored in HBM, then the face pass), for comparison.  The
- * other fluxes use the two-pass kernels in both FAST families. */
+ * kernel (gradients, predictor, faces and update, on chip); FAST_TWO_PASS
+ * keeps the earlier two kernels per stage (gradients and predictor stored in
+ * HBM, then the face pass), for comparison.  The other fluxes use the two-pass
+ * kernels in both FAST families. */
 enum zg_kernels { ZG_KERNELS_PARITY = 0, ZG_KERNELS_FAST = 1, ZG_KERNELS_FAST_TWO_PASS = 2 };
 
 /* Solver configuration: SmFluid(Eos::Ptr) plus its setters
