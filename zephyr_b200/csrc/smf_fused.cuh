@@ -72,9 +72,12 @@ struct FS {
     R r, u, v, p, e, ri;
 };
 
+// half: at the half step's faces
 template <typename R>
-__device__ __forceinline__ R energy_ri(const EosR<R> &eos, R P, R ri, R igm1) {
-    return eos.kind == EOS_IDEAL ? P * ri * igm1 : eos.e0 + (P + eos.gamma * eos.P0) * ri * igm1;
+__device__ __forceinline__ R energy_ri(const EosR<R> &eos, R P, R ri, R igm1, bool half = false) {
+    if (eos.kind == EOS_IDEAL) return rmul(rmul(P, ri), igm1);
+    const R s = half ? radd(P, rmul(eos.gamma, eos.P0)) : rfma(eos.gamma, eos.P0, P);
+    return rfma(rmul(s, ri), igm1, eos.e0);
 }
 
 // models.cpp:58-63 (is_bad) without integer classification: every compare
@@ -87,10 +90,19 @@ __device__ __forceinline__ bool bad_fs(const FS<R> &z, R pmin) {
 }
 
 // phys flux along x of z (models.cpp:131-137 with the normal (1, 0))
+// (k = |v|^2)
+template <typename R>
+__device__ __forceinline__ C4<R> flux_x(const FS<R> &z, R k) {
+    const R ru = rmul(z.r, z.u), E = rfma(R(0.5), k, z.e);
+    return C4<R>{ru, rfma(ru, z.u, z.p), rmul(ru, z.v), rmul(rfma(z.r, E, z.p), z.u)};
+}
 template <typename R>
 __device__ __forceinline__ C4<R> flux_x(const FS<R> &z) {
-    const R ru = z.r * z.u;
-    return C4<R>{ru, ru * z.u + z.p, ru * z.v, (z.r * (z.e + R(0.5) * (z.u * z.u + z.v * z.v)) + z.p) * z.u};
+    return flux_x(z, sq2(z.u, z.v));
+}
+template <typename R>
+__device__ __forceinline__ R sound_ri(const FS<R> &z, const EosR<R> &eos) {
+    return sqrt(rmul(rmul(eos.gamma, radd(z.p, eos.P0)), z.ri));
 }
 
 // HLLC (hllc.cpp:23-83) in the face frame.  hllc.cpp writes the flux in its
@@ -101,16 +113,17 @@ __device__ __forceinline__ C4<R> flux_x(const FS<R> &z) {
 // otherwise.  The kernel evaluates that one side (the two forms agree to
 // rounding), with the side's state chosen before the arithmetic so that a
 // warp runs one path.
-template <typename R>
+// VL, VR: |v|^2 of the left / right state as v^2 + u^2 (see hll_fs).
+template <bool VL, bool VR, typename R>
 __device__ __forceinline__ C4<R> hllc_fs(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
-    const R cL = sqrt(eos.gamma * (L.p + eos.P0) * L.ri), cR = sqrt(eos.gamma * (Rs.p + eos.P0) * Rs.ri);
+    const R cL = sound_ri(L, eos), cR = sound_ri(Rs, eos);
     // (the states are finite here: a NaN ordering of std::min does not arise)
-    const R SL = smin_t(L.u - cL, Rs.u - cR);
-    const R SR = smax_t(L.u + cL, Rs.u + cR);
-    if (SL >= R(0)) return flux_x(L);
-    if (SR <= R(0)) return flux_x(Rs);
-    const R aL = L.r * (SL - L.u), aR = Rs.r * (SR - Rs.u);
-    const R SC = (L.p - Rs.p + aR * Rs.u - aL * L.u) * rcp_r(aR - aL);
+    const R SL = smin_t(rsub(L.u, cL), rsub(Rs.u, cR));
+    const R SR = smax_t(radd(L.u, cL), radd(Rs.u, cR));
+    if (SL >= R(0)) return flux_x(L, VL ? sq2(L.v, L.u) : sq2(L.u, L.v));
+    if (SR <= R(0)) return flux_x(Rs, VR ? sq2(Rs.v, Rs.u) : sq2(Rs.u, Rs.v));
+    const R aL = rmul(L.r, rsub(SL, L.u)), aR = rmul(Rs.r, rsub(SR, Rs.u));
+    const R SC = rmul(rfma(-aL, L.u, rfma(aR, Rs.u, rsub(L.p, Rs.p))), rcp_r(rsub(aR, aL)));
     const bool left = SC >= R(0);
     FS<R> X;
     X.r = left ? L.r : Rs.r;
@@ -119,48 +132,100 @@ __device__ __forceinline__ C4<R> hllc_fs(const FS<R> &L, const FS<R> &Rs, const 
     X.p = left ? L.p : Rs.p;
     X.e = left ? L.e : Rs.e;
     const R SX = left ? SL : SR, aX = left ? aL : aR;
-    const R rs = aX * rcp_r(SX - SC);
-    const R EX = X.e + R(0.5) * (X.u * X.u + X.v * X.v);
-    const R Es = EX + (SC - X.u) * (SC + X.p * rcp_r(aX));
-    const R ru = X.r * X.u;
-    const R rE = X.r * EX;
+    const R rs = rmul(aX, rcp_r(rsub(SX, SC)));
+    const R EX = rfma(R(0.5), sq2(X.u, X.v), X.e);
+    const R Es = rfma(rsub(SC, X.u), rfma(X.p, rcp_r(aX), SC), EX);
+    const R ru = rmul(X.r, X.u);
+    const R rE = rmul(X.r, EX);
     C4<R> f;
-    f.r = ru + SX * (rs - X.r);
-    f.mu = ru * X.u + X.p + SX * (rs * SC - ru);
-    f.mv = ru * X.v + SX * (rs * X.v - X.r * X.v);
-    f.E = (rE + X.p) * X.u + SX * (rs * Es - rE);
+    f.r = rfma(SX, rsub(rs, X.r), ru);
+    f.mu = rfma(SX, rfma(rs, SC, -ru), rfma(ru, X.u, X.p));
+    f.mv = rfma(ru, X.v, rmul(SX, rfma(rs, X.v, -rmul(X.r, X.v))));
+    f.E = rfma(radd(rE, X.p), X.u, rmul(SX, rfma(rs, Es, -rE)));
     return f;
 }
 
-// HLL (hll.cpp:23-57) in the face frame (isolated cells, and the HLL method)
-template <typename R>
+// HLL (hll.cpp:23-57) in the face frame (isolated cells, and the HLL method).
+// VL, VR: |v|^2 of the left / right state as v^2 + u^2; Y: a y face's frame.
+// Interior faces: VR = Y, VL = Y or Heun's first stage; boundary faces: both.
+template <bool VL, bool VR, bool Y, typename R>
 __device__ __forceinline__ C4<R> hll_fs(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
-    const R cL = sqrt(eos.gamma * (L.p + eos.P0) * L.ri), cR = sqrt(eos.gamma * (Rs.p + eos.P0) * Rs.ri);
-    const R SL = smin_t(smin_t(L.u - cL, Rs.u - cR), R(0));
-    const R SR = smax_t(smax_t(L.u + cL, Rs.u + cR), R(0));
-    const C4<R> FL = flux_x(L), FR = flux_x(Rs);
-    const R EL = L.e + R(0.5) * (L.u * L.u + L.v * L.v);
-    const R ER = Rs.e + R(0.5) * (Rs.u * Rs.u + Rs.v * Rs.v);
-    const R QL[4] = {L.r, L.r * L.u, L.r * L.v, L.r * EL};
-    const R QR[4] = {Rs.r, Rs.r * Rs.u, Rs.r * Rs.v, Rs.r * ER};
-    const R fl[4] = {FL.r, FL.mu, FL.mv, FL.E}, fr[4] = {FR.r, FR.mu, FR.mv, FR.E};
-    const R inv = rcp_r(SR - SL), SLR = SL * SR;
-    R o[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o[k] = (SR * fl[k] - SL * fr[k] + SLR * (QR[k] - QL[k])) * inv;
-    return C4<R>{o[0], o[1], o[2], o[3]};
+    const R cL = sound_ri(L, eos), cR = sound_ri(Rs, eos);
+    const R SL = smin_t(smin_t(rsub(L.u, cL), rsub(Rs.u, cR)), R(0));
+    const R SR = smax_t(smax_t(radd(L.u, cL), radd(Rs.u, cR)), R(0));
+    const R EL = rfma(R(0.5), VL ? sq2(L.v, L.u) : sq2(L.u, L.v), L.e);
+    const R ER = rfma(R(0.5), VR ? sq2(Rs.v, Rs.u) : sq2(Rs.u, Rs.v), Rs.e);
+    const R ruL = rmul(L.r, L.u), ruR = rmul(Rs.r, Rs.u), rvL = rmul(L.r, L.v), rvR = rmul(Rs.r, Rs.v);
+    const R inv = rcp_r(rsub(SR, SL)), SLR = rmul(SL, SR);
+    auto mean = [&](R fl, R fr, R dq) { return rmul(rfma(SLR, dq, rfma(SR, fl, -rmul(SL, fr))), inv); };
+    C4<R> o;
+    o.r = mean(ruL, ruR, rsub(Rs.r, L.r));
+    o.mu = mean(rfma(ruL, L.u, L.p), rfma(ruR, Rs.u, Rs.p), rsub(ruR, ruL));
+    o.mv = mean(rmul(ruL, L.v), rmul(ruR, Rs.v), Y ? rfma(-L.r, L.v, rvR) : rfma(Rs.r, Rs.v, -rvL));
+    o.E = mean(rmul(rfma(L.r, EL, L.p), L.u), rmul(rfma(Rs.r, ER, Rs.p), Rs.u), rfma(Rs.r, ER, -rmul(L.r, EL)));
+    return o;
 }
 
 // Limited slope of one component along one axis (see the header comment);
 // inv2h = 1 / 2h, invh = 1 / h.
+// A limiter chosen at run time is out of line: sixteen inlined copies of the
+// switch outgrow the instruction cache (superbee 2nd order at 1400^2: 307 -> 219
+// us a step).
+template <typename R>
+__device__ __noinline__ R limit_rt(int kind, R a, R b) {
+    return lim2<R>(kind, a, b);
+}
 template <int LIM, typename R>
 __device__ __forceinline__ R slope(int kind, R dL, R dR, R inv2h, R invh) {
     if (LIM == LIM_VANALBADA1) {
-        const R p = dL * dR;
+        const R p = rmul(dL, dR);
         if (p >= R(0)) return R(0);
-        return -p * (dR - dL) * rcp_r(dL * dL + dR * dR) * invh;
+        return rmul(rmul(rmul(-p, rsub(dR, dL)), rcp_r(sq2(dL, dR))), invh);
     }
-    return (limit<LIM, R>(kind, -dL, dR) * dR - limit<LIM, R>(kind, -dR, dL) * dL) * inv2h;
+    R a, b;
+    if (LIM >= 0) {
+        a = lim2<R>(LIM, -dL, dR);
+        b = lim2<R>(LIM, -dR, dL);
+    } else {
+        a = limit_rt<R>(kind, -dL, dR);
+        // van Albada 2 is symmetric in its arguments: one value (and one rounding) for both
+        b = kind == LIM_VANALBADA2 ? a : limit_rt<R>(kind, -dR, dL);
+    }
+    if (LIM == LIM_MC || LIM == LIM_MINMOD) return rmul(rfma(-b, dL, rmul(a, dR)), inv2h);
+    return rmul(rfma(a, dR, -rmul(b, dL)), inv2h);
+}
+
+// A cell's value at the face at `off` along an axis (FaceExtra::Direct,
+// face_extra.h:121-184) with slopes g0-g3; low: an interior face on
+// the cell's low side.
+// The energy and 1 / r are the caller's.
+template <typename R>
+__device__ __forceinline__ FS<R> reconstruct(const FS<R> &z, R g0, R g1, R g2, R g3, R off, bool low) {
+    return FS<R>{rfma(g0, off, z.r), low ? radd(z.u, rmul(g1, off)) : rfma(g1, off, z.u),
+                 low ? radd(z.v, rmul(g2, off)) : rfma(g2, off, z.v), rfma(g3, off, z.p), R(0), R(0)};
+}
+// The same at the half step's faces.
+template <typename R>
+__device__ __forceinline__ FS<R> reconstruct_half(const FS<R> &z, const R g[4], R off) {
+    return FS<R>{radd(z.r, rmul(g[0], off)), rfma(g[1], off, z.u), rfma(g[2], off, z.v), radd(z.p, rmul(g[3], off)),
+                 R(0), R(0)};
+}
+
+// A cell's outward flux sum from its faces' fluxes (low x, high x, low y, high y).
+__device__ __forceinline__ double flux_sum(double xl, double xh, double yl, double yh, double hx, double hy) {
+    return rfma(yh, hx, rfma(-yl, hx, rfma(xh, hy, -rmul(xl, hy))));
+}
+
+// Conserved variables of an FP64 primitive state (models.cpp:20-25).
+__device__ __forceinline__ C4<double> cons_of(double r, double u, double v, double e) {
+    return C4<double>{r, r * u, r * v, r * rfma(0.5, sq2(u, v), e)};
+}
+
+// Conserved state of cell ic at t^n.
+template <typename R, bool MIXED>
+__device__ __forceinline__ C4<double> q_n(const Fields<R> &f, int ic) {
+    if (MIXED) return C4<double>{f.q[0][ic], f.q[1][ic], f.q[2][ic], f.q[3][ic]};
+    return cons_of(f.w[0][ic], f.w[1][ic], f.w[2][ic], f.w[4][ic]);
 }
 
 // FP64 primitive state from conserved variables (models.cpp:27-32) with the
@@ -171,8 +236,9 @@ __device__ __forceinline__ P5<double> prim_ri(const C4<double> &q, const EosD &e
     ri = rcp_nr(q.r);
     z.u = q.mu * ri;
     z.v = q.mv * ri;
-    z.e = q.E * ri - 0.5 * (z.u * z.u + z.v * z.v);
-    z.p = eos.kind == EOS_IDEAL ? eos.gm1 * z.r * z.e : eos.gm1 * z.r * (z.e - eos.e0) - eos.gamma * eos.P0;
+    z.e = rfma(q.E, ri, -0.5 * sq2(z.u, z.v));
+    z.p = eos.kind == EOS_IDEAL ? eos.gm1 * z.r * z.e
+                                : rfma(eos.gm1 * z.r, z.e - eos.e0, -rmul(eos.gamma, eos.P0));
     return z;
 }
 
@@ -191,7 +257,7 @@ __device__ __noinline__ C4<R> boundary_flux(FS<R> zm, int s_own, int bc, bool us
     }
     to_local(s_own, zm.u, zm.v);
     to_local(s_own, zp.u, zp.v);
-    C4<R> lf = use_hll ? hll_fs(zm, zp, eos) : hllc_fs(zm, zp, eos);
+    C4<R> lf = use_hll ? hll_fs<true, true, false>(zm, zp, eos) : hllc_fs<true, true>(zm, zp, eos);
     to_global(s_own, lf.mu, lf.mv);
     if (!own_a) {
         lf.r = -lf.r;
@@ -370,8 +436,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                 const int g = gi * m.ny + gj;
                 q0 = C4<double>{f.q[0][g], f.q[1][g], f.q[2][g], f.q[3][g]};
             } else {
-                const double rr = Z[0][zr][zc], u = Z[1][zr][zc], v = Z[2][zr][zc], e = Z[4][zr][zc];
-                q0 = C4<double>{rr, rr * u, rr * v, rr * (e + 0.5 * (u * u + v * v))};
+                q0 = cons_of(Z[0][zr][zc], Z[1][zr][zc], Z[2][zr][zc], Z[4][zr][zc]);
             }
         }
         // boundary flags of the four slots (the normals are the axes)
@@ -411,10 +476,9 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                     const bool ax = s < 2;
                     const R off = s == 0 ? -halfx : (s == 1 ? halfx : (s == 2 ? -halfy : halfy));
                     const R *gg = ax ? gx : gy;
-                    FS<R> zm{zc5.r + gg[0] * off, zc5.u + gg[1] * off, zc5.v + gg[2] * off, zc5.p + gg[3] * off,
-                             R(0), R(0)};
+                    FS<R> zm = reconstruct_half(zc5, gg, off);
                     zm.ri = rcp_r(zm.r);
-                    zm.e = energy_ri(eos, zm.p, zm.ri, igm1);
+                    zm.e = energy_ri(eos, zm.p, zm.ri, igm1, true);
                     if (bad_fs(zm, eos.pmin)) zm = zc5;
                     C4<R> lf;
                     if (ax) {
@@ -469,12 +533,12 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
     // reconstruction of G cell (gr, gc) at its face on axis `ax` (0: x, 1: y),
     // side `hi` (the +x / +y face, else the low one), FaceExtra::Direct
     // (face_extra.h:121-184); a bad value falls back to the cell state
-    auto recon = [&](int gr, int gc, int ax, bool hi) {
+    auto recon = [&](int gr, int gc, int ax, bool hi, bool boundary) {
         const FS<R> z = sc(gr, gc);
         const R off = ax == 0 ? (hi ? halfx : -halfx) : (hi ? halfy : -halfy);
         const int b = 4 * ax;
-        FS<R> o{z.r + G[b][gr][gc] * off, z.u + G[b + 1][gr][gc] * off, z.v + G[b + 2][gr][gc] * off,
-                z.p + G[b + 3][gr][gc] * off, R(0), R(0)};
+        FS<R> o = reconstruct(z, G[b][gr][gc], G[b + 1][gr][gc], G[b + 2][gr][gc], G[b + 3][gr][gc], off,
+                              !hi && !boundary);
         o.ri = rcp_r(o.r);
         o.e = energy_ri(eos, o.p, o.ri, igm1);
         if (bad_fs(o, eos.pmin)) {
@@ -494,8 +558,8 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
             zm = sc_ri(r, l);
             zp = sc_ri(rB, lB);
         } else {
-            zm = recon(r, l, DIR, true);
-            zp = recon(rB, lB, DIR, false);
+            zm = recon(r, l, DIR, true, false);
+            zp = recon(rB, lB, DIR, false, false);
         }
         if (DIR == 1) {
             R t = zm.u;
@@ -505,7 +569,8 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
             zp.u = zp.v;
             zp.v = -t;
         }
-        C4<R> lf = (robust || a.flux == FLUX_HLL) ? hll_fs(zm, zp, eos) : hllc_fs(zm, zp, eos);
+        constexpr bool VR = DIR == 1, VL = VR || MODE == FUSED_HEUN_A;
+        C4<R> lf = (robust || a.flux == FLUX_HLL) ? hll_fs<VL, VR, DIR == 1>(zm, zp, eos) : hllc_fs<VL, VR>(zm, zp, eos);
         if (DIR == 1) {
             const R t = lf.mu;
             lf.mu = -lf.mv;
@@ -518,8 +583,8 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
         const int gr = own_a ? r : r + (dir == 0), gc = own_a ? l : l + (dir == 1);
         const int s_own = own_a ? (dir == 0 ? 1 : 3) : (dir == 0 ? 0 : 2);
         const bool robust = PC && wt[gr][gc];
-        const FS<R> zm = robust ? sc_ri(gr, gc) : recon(gr, gc, dir, own_a);
-        return boundary_flux<R>(zm, s_own, m.bc[s_own], robust || a.flux == FLUX_HLL, eos, own_a);
+        const FS<R> zm = robust ? sc_ri(gr, gc) : recon(gr, gc, dir, own_a, true);
+        return boundary_flux(zm, s_own, m.bc[s_own], robust || a.flux == FLUX_HLL, eos, own_a);
     };
     // (predictor-corrector: the fluxes overwrite Z, which no thread reads
     // after phase 1)
@@ -555,24 +620,22 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
         double F[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            F[k] = ((-FX[k][r - 1][l] * hy + FX[k][r][l] * hy) - FY[k][r - 1][l - 1] * hx) + FY[k][r - 1][l] * hx;
+            F[k] = flux_sum(FX[k][r - 1][l], FX[k][r][l], FY[k][r - 1][l - 1], FY[k][r - 1][l], hx, hy);
         C4<double> q;
         if (PC) {
             q = C4<double>{Q[0][r][l], Q[1][r][l], Q[2][r][l], Q[3][r][l]};
         } else if (MODE == FUSED_HEUN_B) {
             // Q(z*) of the stage value
-            const double rr = Z[0][r + 1][l + 1], u = Z[1][r + 1][l + 1], v = Z[2][r + 1][l + 1],
-                         e = Z[4][r + 1][l + 1];
-            q = C4<double>{rr, rr * u, rr * v, rr * (e + 0.5 * (u * u + v * v))};
+            q = cons_of(Z[0][r + 1][l + 1], Z[1][r + 1][l + 1], Z[2][r + 1][l + 1], Z[4][r + 1][l + 1]);
         } else {
-            q = q_of<R, MIXED>(f, ic);
+            q = q_n<R, MIXED>(f, ic);
         }
         q.r -= coef * F[0];
         q.mu -= coef * F[1];
         q.mv -= coef * F[2];
         q.E -= coef * F[3];
         if (MODE == FUSED_HEUN_B) {
-            const C4<double> q0 = q_of<R, MIXED>(f, ic);
+            const C4<double> q0 = q_n<R, MIXED>(f, ic);
             q.r = 0.5 * (q0.r + q.r);
             q.mu = 0.5 * (q0.mu + q.mu);
             q.mv = 0.5 * (q0.mv + q.mv);
@@ -589,7 +652,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                     // isolation (sm_fluid.cpp:354-358): keep the old state
                     zn = P5<double>{(double)f.w[0][ic], (double)f.w[1][ic], (double)f.w[2][ic],
                                     (double)f.w[3][ic], (double)f.w[4][ic]};
-                    q = q_of<R, MIXED>(f, ic);
+                    q = q_n<R, MIXED>(f, ic);
                     ri = rcp_nr(zn.r);
                     wn = 3;
                 } else if (wn > 0) {
@@ -604,8 +667,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                 f.qn[3][ic] = q.E;
             }
             st5(f.wn, ic, down<R>(zn));
-            low = cfl_lower(smin(m.inc2x[i], m.inc2y[j]), a.eos.gamma * (zn.p + a.eos.P0) * ri,
-                            zn.u * zn.u + zn.v * zn.v);
+            low = cfl_lower(smin(m.inc2x[i], m.inc2y[j]), a.eos.gamma * (zn.p + a.eos.P0) * ri, sq2(zn.u, zn.v));
         }
     }
     // The minimum of the CFL terms of the new state for the next step
@@ -629,9 +691,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
         if (__any_sync(0xffffffffu, take)) {
             unsigned long long best = 0x7FEFFFFFFFFFFFFFull;
             if (take) {
-                const double c = sqrt(a.eos.gamma * (zn.p + a.eos.P0) / zn.r);
-                const double dinc = sqrt(smin(m.inc2x[i], m.inc2y[j]));
-                const double lam = dinc / (sqrt(zn.u * zn.u + zn.v * zn.v) + c);
+                const double lam = cfl_term(a, i, j, zn.r, zn.u, zn.v, zn.p, MIXED && PC);
                 if (lam >= 0.0) best = dbits(lam);
             }
             for (int o = 16; o > 0; o >>= 1) {

@@ -20,9 +20,13 @@
 // with 4 warps per scheduler (128 registers).  Two things that cost more than
 // they look: an atomic minimum per cell on the one CFL slot (190 us at 1024^2
 // against 88 with one per warp), and bad-value fallbacks as selects instead of
-// branches under a warp vote (317 against 301 us at 2048^2).
-// Measured (B200, one step, FP64 / MIXED): 2048^2 predictor-corrector 354 ->
-// 314 / 294 -> 250 us, Heun 541 -> 430 / 470 -> 321 us.
+// branches under a warp vote (5 % of a step at 2048^2).
+// Measured (B200, one step, FP64 / MIXED): 2048^2 predictor-corrector 353 ->
+// 310 / 293 -> 247 us, Heun 542 -> 430 / 457 -> 305 us.
+// MIXED gives the tile's bits: the same FP32 formulas with their roundings
+// written out (smf_tiled.cuh), the same order of the flux sum.  That holds on
+// periodic axes; a boundary face is another instance in the tile (seen from its
+// own cell), so MIXED marches only on rectangles that are periodic both ways.
 #pragma once
 
 #include "smf_fused.cuh"
@@ -60,8 +64,9 @@ __device__ __forceinline__ bool bad_rp(double r, double p, double pmin) {
 // face_extra.h:121-184) with slopes gr; the cell's own state where that is
 // bad.  All lanes of the warp call it.
 template <typename R>
-__device__ __forceinline__ FS<R> face_value(const FS<R> &h, const R gr[4], R off, const EosR<R> &eos, R igm1) {
-    FS<R> o{h.r + gr[0] * off, h.u + gr[1] * off, h.v + gr[2] * off, h.p + gr[3] * off, R(0), R(0)};
+__device__ __forceinline__ FS<R> face_value(const FS<R> &h, const R gr[4], R off, bool low, const EosR<R> &eos,
+                                            R igm1) {
+    FS<R> o = reconstruct(h, gr[0], gr[1], gr[2], gr[3], off, sizeof(R) == 4 && low);
     o.ri = rcp_r(o.r);
     o.e = energy_ri(eos, o.p, o.ri, igm1);
     bool b;
@@ -103,9 +108,9 @@ __device__ __forceinline__ FS<R> half_step(const FS<R> &c, const C4<double> &q0,
             lf.mv = ax ? rn * v : rn * v + p;
             lf.E = (re + 0.5 * r * (u * u + v * v) + p) * n;
         } else {
-            FS<R> zm{c.r + gg[0] * off, c.u + gg[1] * off, c.v + gg[2] * off, c.p + gg[3] * off, R(0), R(0)};
+            FS<R> zm = reconstruct_half(c, gg, off);
             zm.ri = rcp_r(zm.r);
-            zm.e = energy_ri(eos, zm.p, zm.ri, k.igm1);
+            zm.e = energy_ri(eos, zm.p, zm.ri, k.igm1, true);
             rare(bad_fs(zm, eos.pmin), [&] { zm = c; });
             if (ax) {
                 lf = flux_x(zm);
@@ -162,12 +167,11 @@ __device__ __forceinline__ C4<double> hllc_march(const FS<double> &L, const FS<d
     }
     return f;
 }
-__device__ __forceinline__ C4<float> hllc_march(const FS<float> &L, const FS<float> &Rs, const EosR<float> &eos) {
-    return hllc_fs(L, Rs, eos);
-}
-template <bool HLL, typename R>
+// VL, VR, Y: as hll_fs
+template <bool HLL, bool VL, bool VR, bool Y, typename R>
 __device__ __forceinline__ C4<R> march_flux(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
-    if constexpr (HLL) return hll_fs(L, Rs, eos);
+    if constexpr (HLL) return hll_fs<VL, VR, Y>(L, Rs, eos);
+    else if constexpr (sizeof(R) == 4) return hllc_fs<VL, VR>(L, Rs, eos);
     else return hllc_march(L, Rs, eos);
 }
 
@@ -185,18 +189,17 @@ struct WarpCfl {
     __device__ __forceinline__ void refresh(const unsigned long long *slot) {
         reported = __double2float_ru(__longlong_as_double((long long)__ldcg(slot)));
     }
-    // all lanes of the warp call it; `live`: with a cell
+    // all lanes of the warp call it; `live`: with a cell; VU: as cfl_term's vu
+    template <bool VU>
     __device__ __forceinline__ void add(const SmfArgs &a, int i, int j, const P5<double> &z, double ri, bool live) {
         const StructMesh &m = a.mesh;
-        const float lo = cfl_lower(m.inc2min, a.eos.gamma * (z.p + a.eos.P0) * ri, z.u * z.u + z.v * z.v);
+        const float lo = cfl_lower(m.inc2min, a.eos.gamma * (z.p + a.eos.P0) * ri, sq2(z.u, z.v));
         // (bounds are >= 0, so they order like their bits)
         const float w = live && lo > 0.0f ? lo : INFINITY;
         low = fminf(low, __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(w))));
         // 1.0005: a bound is at most 3e-4 below its term
         if (live && lo <= fminf(low * 1.0005f, reported)) {
-            const double c = sqrt(a.eos.gamma * (z.p + a.eos.P0) / z.r);
-            const double dinc = sqrt(smin(m.inc2x[i], m.inc2y[j]));
-            const double lam = dinc / (sqrt(z.u * z.u + z.v * z.v) + c);
+            const double lam = cfl_term(a, i, j, z.r, z.u, z.v, z.p, VU);
             if (lam >= 0.0 && dbits(lam) < best) best = dbits(lam);
         }
     }
@@ -228,7 +231,7 @@ __device__ __forceinline__ void store_cell(const SmfArgs &a, const Fields<R> &f,
                 // isolation (sm_fluid.cpp:354-358): keep the old state
                 zn = P5<double>{(double)f.w[0][ic], (double)f.w[1][ic], (double)f.w[2][ic], (double)f.w[3][ic],
                                 (double)f.w[4][ic]};
-                q = q_of<R, MIXED>(f, ic);
+                q = q_n<R, MIXED>(f, ic);
                 ri = rcp_nr(zn.r);
                 wn = 3;
             } else if (wn > 0) {
@@ -244,7 +247,7 @@ __device__ __forceinline__ void store_cell(const SmfArgs &a, const Fields<R> &f,
         }
         st5(f.wn, ic, down<R>(zn));
     }
-    cfl.add(a, i, j, zn, ri, live);
+    cfl.add<MIXED && MODE == FUSED_PC>(a, i, j, zn, ri, live);
 }
 
 // One asynchronous copy of a lane's value (4 or 8 bytes) into shared memory.
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                                                                   const __grid_constant__ Fields<R> f,
                                                                   const __grid_constant__ StepConst<R> k, int strips,
                                                                   int rows) {
-    constexpr bool PC = MODE == FUSED_PC;
+    constexpr bool PC = MODE == FUSED_PC, FIRST = MODE == FUSED_HEUN_A;
     constexpr unsigned ALL = 0xffffffffu;
     using Ring = MarchRing<R, MIXED, MODE>;
     __shared__ Ring rings[MARCH_WARPS];
@@ -326,9 +329,6 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
             }
         }
     };
-    auto cons_of = [](double r, double u, double v, double e) {
-        return C4<double>{r, r * u, r * v, r * (e + 0.5 * (u * u + v * v))};
-    };
     // conserved state at t^n of the row in slot sb of the base ring (slot sz of the state ring)
     auto base = [&](int sz, int sb) {
         if constexpr (Ring::BASE) {
@@ -341,7 +341,11 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
     };
 
     FS<R> up{};     // row g - 1's state at its high face
-    double acc[4];  // row g - 1: the fluxes through its other three faces
+    // row g - 1: the fluxes through its other three faces.  FP64: their sum.
+    // MIXED: the FP32 fluxes themselves (low x, low y, high y), summed in the
+    // tile's order, so that both forms give the same bits
+    double acc[4];
+    C4<R> fxl{}, fyl{}, fyh{};
     int sm = 0, sc = 1, sp = 2, sn = 3;  // state slots of rows g - 1, g, g + 1, g + 2
     int bm = 2, bc = 0, bp = 1;          // base slots of rows g - 1, g, g + 1
     fetch_z(i_lo - 2, sm);
@@ -402,8 +406,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
         // ---- faces between lanes l and l + 1 (frame of the +y normal) ------
         C4<R> fy;
         {
-            FS<R> L = face_value<R>(h, gy, k.halfy, eos, k.igm1);
-            FS<R> Rs = shfl_down_fs(face_value<R>(h, gy, -k.halfy, eos, k.igm1));
+            FS<R> L = face_value<R>(h, gy, k.halfy, false, eos, k.igm1);
+            FS<R> Rs = shfl_down_fs(face_value<R>(h, gy, -k.halfy, true, eos, k.igm1));
             bool robust = false;
             if (iso) {
                 const FS<R> next = shfl_down_fs(own);
@@ -421,14 +425,14 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 }
             }
             const FS<R> Ln{L.r, L.v, L.u, L.p, L.e, L.ri}, Rn{Rs.r, Rs.v, Rs.u, Rs.p, Rs.e, Rs.ri};
-            C4<R> t = march_flux<HLL, R>(Ln, Rn, eos);
-            if (!HLL && robust) t = hll_fs(Ln, Rn, eos);
+            C4<R> t = march_flux<HLL, true, true, true, R>(Ln, Rn, eos);
+            if (!HLL && robust) t = hll_fs<true, true, true>(Ln, Rn, eos);
             fy = C4<R>{t.r, t.mv, t.mu, t.E};
         }
         // ---- faces between rows g - 1 and g -------------------------------
         C4<R> fx{};
         if (g > i_lo - 1) {
-            FS<R> L = up, Rs = face_value<R>(h, gx, -k.halfx, eos, k.igm1);
+            FS<R> L = up, Rs = face_value<R>(h, gx, -k.halfx, true, eos, k.igm1);
             const bool robust = iso && (wm | wc) != 0;
             if (robust) Rs = own;
             if (low) {
@@ -439,8 +443,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 Rs = L;
                 if (m.bc[1] == BC_WALL) Rs.u = -Rs.u;
             }
-            fx = march_flux<HLL, R>(L, Rs, eos);
-            if (!HLL && robust) fx = hll_fs(L, Rs, eos);
+            fx = march_flux<HLL, FIRST, false, false, R>(L, Rs, eos);
+            if (!HLL && robust) fx = hll_fs<FIRST, false, false>(L, Rs, eos);
         }
         // ---- update of row g - 1 -------------------------------------------
         if (g > i_lo) {
@@ -449,10 +453,17 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
             C4<double> q = MODE == FUSED_HEUN_B
                                ? cons_of(ring.z[sm][0][l], ring.z[sm][1][l], ring.z[sm][2][l], ring.z[sm][4][l])
                                : base(sm, bm);
-            q.r -= coef * (acc[0] + (double)fx.r * hy);
-            q.mu -= coef * (acc[1] + (double)fx.mu * hy);
-            q.mv -= coef * (acc[2] + (double)fx.mv * hy);
-            q.E -= coef * (acc[3] + (double)fx.E * hy);
+            if constexpr (MIXED) {
+                q.r -= coef * flux_sum(fxl.r, fx.r, fyl.r, fyh.r, hx, hy);
+                q.mu -= coef * flux_sum(fxl.mu, fx.mu, fyl.mu, fyh.mu, hx, hy);
+                q.mv -= coef * flux_sum(fxl.mv, fx.mv, fyl.mv, fyh.mv, hx, hy);
+                q.E -= coef * flux_sum(fxl.E, fx.E, fyl.E, fyh.E, hx, hy);
+            } else {
+                q.r -= coef * (acc[0] + (double)fx.r * hy);
+                q.mu -= coef * (acc[1] + (double)fx.mu * hy);
+                q.mv -= coef * (acc[2] + (double)fx.mv * hy);
+                q.E -= coef * (acc[3] + (double)fx.E * hy);
+            }
             if (MODE == FUSED_HEUN_B) {
                 const C4<double> qn = base(sm, bm);
                 q.r = 0.5 * (qn.r + q.r);
@@ -465,11 +476,15 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
         // ---- carry row g over -----------------------------------------------
         const C4<R> fb{__shfl_up_sync(ALL, fy.r, 1), __shfl_up_sync(ALL, fy.mu, 1), __shfl_up_sync(ALL, fy.mv, 1),
                        __shfl_up_sync(ALL, fy.E, 1)};
-        acc[0] = (-(double)fx.r * hy - (double)fb.r * hx) + (double)fy.r * hx;
-        acc[1] = (-(double)fx.mu * hy - (double)fb.mu * hx) + (double)fy.mu * hx;
-        acc[2] = (-(double)fx.mv * hy - (double)fb.mv * hx) + (double)fy.mv * hx;
-        acc[3] = (-(double)fx.E * hy - (double)fb.E * hx) + (double)fy.E * hx;
-        up = face_value<R>(h, gx, k.halfx, eos, k.igm1);
+        if constexpr (MIXED) {
+            fxl = fx, fyl = fb, fyh = fy;
+        } else {
+            acc[0] = (-(double)fx.r * hy - (double)fb.r * hx) + (double)fy.r * hx;
+            acc[1] = (-(double)fx.mu * hy - (double)fb.mu * hx) + (double)fy.mu * hx;
+            acc[2] = (-(double)fx.mv * hy - (double)fb.mv * hx) + (double)fy.mv * hx;
+            acc[3] = (-(double)fx.E * hy - (double)fb.E * hx) + (double)fy.E * hx;
+        }
+        up = face_value<R>(h, gx, k.halfx, false, eos, k.igm1);
         if (iso && (wc | wp) != 0) up = own;
         wm = wc;
         wc = wp;

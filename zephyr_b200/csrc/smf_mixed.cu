@@ -113,7 +113,7 @@ void launch_step(const SmfArgs &a, const Fields<float> &f, int mode, void *strea
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_MIXED_MARCH_MINB);
     constexpr int TH = ZG_MIXED_FUSED_TH;
     const long long tiles = (long long)((a.mesh.ny + 29) / 30) * ((a.mesh.nx + TH - 1) / TH);
-    if (tiled::march_limiter(a.limiter) &&
+    if (tiled::march_limiter(a.limiter) && a.mesh.xper && a.mesh.yper &&
         sp.rows >= (mode == tiled::FUSED_PC ? MARCH_MIN_ROWS_PC : MARCH_MIN_ROWS_HEUN))
         tiled::march_dispatch<float, true, ZG_MIXED_MARCH_MINB>(a, f, mode, sp, s);
     else if (4 * tiles <= 3 * 148)

@@ -365,17 +365,43 @@ __device__ inline void face_offset(const Fields<R> &f, int i, int j, int s, R &d
 }
 
 // Slope limiter phi(a, b): LIM >= 0 fixes the limiter at compile time, -1
-// selects it at run time: out of line, because sixteen inlined copies of the
-// switch outgrow the instruction cache (superbee 2nd order at 1400^2: 307 -> 219
-// us a step).
-template <typename R>
-__device__ __noinline__ R limit_rt(int kind, R a, R b) {
-    return lim2<R>(kind, a, b);
-}
+// selects it at run time.
 template <int LIM, typename R>
 __device__ inline R limit(int kind, R a, R b) {
-    if constexpr (LIM >= 0) return lim2<R>(LIM, a, b);
-    else return limit_rt<R>(kind, a, b);
+    return lim2<R>(LIM >= 0 ? LIM : kind, a, b);
+}
+
+// Arithmetic with its roundings written out.  Left to the compiler, which of
+// two products of a sum goes into a fused multiply-add depends on the code
+// around it, and these formulas are compiled many times (tiles of two heights,
+// interior and border tiles, the march): two blocks then add different fluxes
+// to the two cells of the face between them, and a state's result depends on
+// where it lies in the mesh (one step of HLL: up to 4e-7 of a field in FP32).
+// With these, every copy gives the same bits.  The choices in each formula
+// (which product is rounded; `low` in reconstruct, `half` in energy_ri, VL and
+// VR in hll_fs) are those that the one tile kernel of 14 rows was compiled to
+// when it ran every mesh, so that MIXED results stay what they were.
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double rsub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+// u^2 + v^2
+template <typename R>
+__device__ __forceinline__ R sq2(R u, R v) {
+    return rfma(u, u, rmul(v, v));
+}
+
+// A cell's CFL term (sm_fluid.cpp:104-111).  vu: |v|^2 as v^2 + u^2 (the MIXED
+// predictor-corrector; the others agree with k_cfl to the bit, so that slabs,
+// which run k_cfl every step, take the single domain's dt).
+__device__ __forceinline__ double cfl_term(const SmfArgs &a, int i, int j, double rho, double u, double v, double p,
+                                           bool vu = false) {
+    const double c = sqrt(a.eos.gamma * (p + a.eos.P0) / rho);
+    return sqrt(smin(a.mesh.inc2x[i], a.mesh.inc2y[j])) / (sqrt(vu ? sq2(v, u) : sq2(u, v)) + c);
 }
 
 template <typename R>
@@ -786,9 +812,7 @@ __global__ void __launch_bounds__(BLOCK) k_cfl(SmfArgs a, Fields<R> f) {
         } else {
             rho = f.w[0][ic], u = f.w[1][ic], v = f.w[2][ic], p = f.w[3][ic];
         }
-        double c = sqrt(a.eos.gamma * (p + a.eos.P0) / rho);
-        double dinc = sqrt(smin(m.inc2x[i], m.inc2y[j]));
-        double lam = dinc / (sqrt(u * u + v * v) + c);
+        const double lam = cfl_term(a, i, j, rho, u, v, p);
         if (lam >= 0.0) best = dbits(lam);
     }
     for (int o = 16; o > 0; o >>= 1) {
