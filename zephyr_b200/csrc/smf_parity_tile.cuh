@@ -44,7 +44,7 @@ struct Args {
     Axis x, y;
     PrimPtr zin, zout;      // source and result of the stage
     const double *dt_in;    // this step's dt
-    double *dt_next;        // the next step's (last stage)
+    double *dt_next;        // the next step's (last stage; null: not asked for)
 };
 
 // Physical flux along an axis of a state with normal velocity n, tangential t
@@ -515,7 +515,7 @@ __device__ __forceinline__ void tile(const Args &A) {
             low = ok ? __fdividef(d, s) * 0.9998f : 0.0f;
         }
     }
-    if (MODE == HEUN_A) return;
+    if (MODE == HEUN_A || !A.dt_next) return;
     // The next step's dt (compute_dt, sm_fluid.cpp:104-116), k_dt's arithmetic;
     // the term is formed only where its lower bound does not exceed the
     // block's smallest (1.0005: a bound is at most 3e-4 below its term).

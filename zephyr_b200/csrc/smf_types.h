@@ -118,7 +118,7 @@ enum : int { PC = 1, HEUN_A = 2, HEUN_B = 3 };
 namespace parity {
 // One second-order stage (ptile::PC ... HEUN_B) of a rectangle with HLLC or HLL in one
 // kernel: zin -> zout at the dt in *dt_in; the last stage leaves the next dt
-// in *dt_next.
+// in *dt_next (where set).
 void launch_tile(const SmfArgs &a, const ptile::Axis &x, const ptile::Axis &y, int stage, PrimPtr zin, PrimPtr zout,
                  const double *dt_in, double *dt_next, void *stream);
 void launch_dt(const SmfArgs &a, PrimPtr z, bool slots, void *stream);

@@ -93,6 +93,10 @@ struct zg_ctx {
     double *d_dt = nullptr;     // dt of the last step
     double *d_dt2 = nullptr;    // the other dt slot: the next step's dt when dt_next_ready
     bool dt_next_ready = false; // the last step (FAST adaptive, PARITY) left the next dt in d_dt2
+    // A step or an upload was recorded into a graph: a replay changes the state
+    // and the dt unseen by the host, so from then on every PARITY step takes
+    // its own dt, into the slot that the recorded ones write.
+    bool recorded = false;
     int *d_flags = nullptr;
     PrimPtr z{}, zhalf{}, znext{};
     double *gx[4] = {}, *gy[4] = {};
@@ -216,6 +220,7 @@ void free_solver(zg_ctx *c) {
     c->d_dt = nullptr;
     c->d_dt2 = nullptr;
     c->dt_next_ready = false;
+    c->recorded = false;
     c->d_flags = nullptr;
     c->configured = false;
     c->stepped = false;
@@ -579,23 +584,24 @@ bool parity_tiles(const zg_ctx *c) {
     return !c->slots && c->par.accuracy == 2 && (c->par.flux == ZG_FLUX_HLLC || c->par.flux == ZG_FLUX_HLL);
 }
 
+// The state is about to be changed on the context's stream: is that recorded?
+void note_recording(zg_ctx *c) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) c->recorded = true;
+}
+
 // One step of SmFluid::update (sm_fluid.cpp:81-102) as kernel launches, bit
 // for bit.  The step's last kernel also takes the dt of the state it writes,
 // into the other dt slot; a dt pass runs only after the state came from
-// elsewhere.
+// elsewhere, and always once a step was recorded.
 int enqueue_parity_step(zg_ctx *c) {
     if (c->par.accuracy == 2) c->grad_ordered = false;  // this step's gradients, in the mesh's order
     void *st = (void *)c->stream;
-    // A recorded step runs again on states it does not know: it brings its own
-    // dt pass, and leaves no minimum that a later step could take as computed.
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(c->stream, &cs);
-    const bool live = cs == cudaStreamCaptureStatusNone;
-    const bool have_dt = c->dt_next_ready && live, pc = c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR;
+    const bool have_dt = c->dt_next_ready && !c->recorded, pc = c->par.scheme == ZG_SCHEME_PREDICTOR_CORRECTOR;
     if (have_dt) std::swap(c->d_dt, c->d_dt2);
     SmfArgs a = make_args(c);
     if (!have_dt) timed(c, ZG_K_DT, [&] { parity::launch_dt(a, c->z, c->slots, st); });
-    double *next = c->d_dt2;
+    double *next = c->recorded ? nullptr : c->d_dt2;
     auto tile = [&](int kind, int stage, PrimPtr zin, PrimPtr zout) {
         timed(c, kind, [&] { parity::launch_tile(a, c->pax, c->pay, stage, zin, zout, c->d_dt, next, st); });
     };
@@ -620,7 +626,7 @@ int enqueue_parity_step(zg_ctx *c) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "kernel launch");
     std::swap(c->z, c->znext);  // Storage::swap of init and next (sm_fluid.cpp:368-370)
-    c->dt_next_ready = live;
+    c->dt_next_ready = next != nullptr;
     c->cfl_valid = false;
     c->stepped = true;
     return ZG_OK;
@@ -899,6 +905,7 @@ int enqueue_slot_mixed_step(zg_ctx *c) {
 }
 
 int enqueue_step(zg_ctx *c) {
+    note_recording(c);
     const bool fast = c->par.kernels != ZG_KERNELS_PARITY;
     if (c->smesh.vol_alt && (fast || c->par.precision != ZG_FP64 || (c->par.accuracy == 2 &&
                                                                         c->par.scheme == ZG_SCHEME_HEUN)))
@@ -1323,6 +1330,7 @@ int zg_state_upload(zg_ctx *c, const double *rho, const double *vx, const double
     DeviceGuard g(c->device);
     int rc = leave_order(c);  // the counters held in the cell order come back with it
     if (rc != ZG_OK) return rc;
+    note_recording(c);
     size_t bytes = (size_t)c->n * sizeof(double);
     const double *src[5] = {rho, vx, vy, p, e};
     double *dst[5] = {c->z.r, c->z.u, c->z.v, c->z.p, c->z.e};
