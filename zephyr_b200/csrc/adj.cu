@@ -47,6 +47,7 @@
 
 #include "../../include/zephyr_gpu.h"
 #include "adj_math.cuh"
+#include "row_grid.h"
 
 namespace zg {
 namespace adj {
@@ -175,7 +176,8 @@ __global__ void __launch_bounds__(32 * (STH + 2), 2) k_stage(Grid g, CF4 X, doub
     extern __shared__ __align__(16) unsigned char stage_smem[];
     StageShm<S> &sm = *reinterpret_cast<StageShm<S> *>(stage_smem);
     const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l;
-    const int i0 = blockIdx.y * STH, j0 = blockIdx.x * 30;
+    const int i0 = (blockIdx.z * gridDim.y + blockIdx.y) * STH, j0 = blockIdx.x * 30;
+    if (i0 >= g.nx) return;
     for (int k = tid; k < (STH + 4) * 34; k += 32 * (STH + 2)) {
         const int zr = k / 34, zc = k - zr * 34;
         double w[4];
@@ -659,7 +661,7 @@ void stage(zg_adj *a, cudaStream_t st, const zg_adj_params &p, const F4 &X, cons
         if (a->device < 64) attr_set |= 1ull << a->device;
     }
     const WG wg = keep ? *keep : WG{};
-    const dim3 grid((unsigned)((a->g.ny + 29) / 30), (unsigned)((a->g.nx + STH - 1) / STH));
+    const dim3 grid = zg::row_grid((unsigned)((a->g.ny + 29) / 30), (unsigned)((a->g.nx + STH - 1) / STH));
     k_stage<S><<<grid, dim3(32, STH + 2), sizeof(StageShm<S>), st>>>(
         a->g, cf(X), p.gamma, 1.0 / (p.gamma - 1.0), p.limiter_eps, base, alpha, beta, p.dt / a->g.vol, keep != nullptr,
         wg.W, as<S>(wg.gx), as<S>(wg.gy), out);

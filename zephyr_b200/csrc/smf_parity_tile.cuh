@@ -214,8 +214,9 @@ __device__ __forceinline__ int wrap(int x, int n) {
 
 // One block's tile.  INTERIOR: the staged region lies inside the mesh, so the
 // boundary selects and the wrapping drop out.
+// (i0, j0): its first row and column.
 template <int MODE, int LIM, bool HLL, int TH, bool INTERIOR>
-__device__ __forceinline__ void tile(const Args &A) {
+__device__ __forceinline__ void tile(const Args &A, int i0, int j0) {
     using L = Layout<MODE, TH>;
     constexpr int ZR = L::ZR, ZC = L::ZC, GR = L::GR, NT = L::NT, HALO = L::H;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -232,7 +233,6 @@ __device__ __forceinline__ void tile(const Args &A) {
     const StructMesh &m = a.mesh;
     const EosD &eos = a.eos;
     const int l = threadIdx.x, r = threadIdx.y, tid = r * 32 + l;
-    const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
 
     // ---- stage the state ------------------------------------------------------
     if (INTERIOR) {
@@ -543,7 +543,7 @@ __device__ __forceinline__ void tile(const Args &A) {
     if (tid == 0) {
         __threadfence();
         const unsigned int ticket = atomicAdd(a.dt_ticket, 1u);
-        if (ticket == gridDim.x * gridDim.y - 1) {  // no block waits for another
+        if (ticket == gridDim.x * (unsigned)((m.nx + TH - 1) / TH) - 1) {  // no block waits for another
             const unsigned long long bits = atomicMin(a.dmin_bits, 0x7FEFFFFFFFFFFFFFull);
             *A.dt_next = smin(a.CFL * __longlong_as_double((long long)bits), a.max_dt);
             *a.dmin_bits = 0x7FEFFFFFFFFFFFFFull;
@@ -557,15 +557,16 @@ template <int MODE, int LIM, bool HLL, int TH, int MINB>
 __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_tile(const __grid_constant__ Args A) {
     after_previous();
     constexpr int H = Layout<MODE, TH>::H;
-    const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
+    const int i0 = (blockIdx.z * gridDim.y + blockIdx.y) * TH, j0 = blockIdx.x * 30;
+    if (i0 >= A.a.mesh.nx) return;
     // (a limiter chosen at run time: one copy of its code)
     if constexpr (LIM >= 0) {
         if (i0 >= H && i0 + TH + H <= A.a.mesh.nx && j0 >= H && j0 + 30 + H <= A.a.mesh.ny) {
-            tile<MODE, LIM, HLL, TH, true>(A);
+            tile<MODE, LIM, HLL, TH, true>(A, i0, j0);
             return;
         }
     }
-    tile<MODE, LIM, HLL, TH, false>(A);
+    tile<MODE, LIM, HLL, TH, false>(A, i0, j0);
 }
 
 template <int MODE, int LIM, bool HLL, int TH, int MINB>
@@ -580,7 +581,7 @@ inline void launch(const Args &A, cudaStream_t s) {
         if (dev < 64) attr_set |= 1ull << dev;
     }
     const StructMesh &m = A.a.mesh;
-    launch_after(kern, dim3((m.ny + 29) / 30, (m.nx + TH - 1) / TH), dim3(32, TH + 2), L::bytes, s, A);
+    launch_after(kern, row_grid((m.ny + 29) / 30, (m.nx + TH - 1) / TH), dim3(32, TH + 2), L::bytes, s, A);
 }
 
 }  // namespace ptile

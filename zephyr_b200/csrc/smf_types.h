@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include "row_grid.h"
 #include "smf_math.cuh"
 
 namespace zg {
