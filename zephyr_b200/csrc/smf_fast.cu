@@ -99,6 +99,8 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
 // so the march from 16 rows per segment on (1024^2).  Below, the tile kernel;
 // where its grid would leave a quarter of the SMs without a block, tiles of 2
 // rows instead of 14 (64^2 10.7 -> 8.7 us, 200^2 11.3 -> 10.9, 256^2 15 -> 17).
+// All forms give the same bits, so that the slabs of a mesh may each take the
+// form of their own size.
 constexpr int MARCH_MIN_ROWS_PC = 16, MARCH_MIN_ROWS_HEUN = 16;
 void launch_step(const SmfArgs &a, const Fields<double> &f, int mode, void *stream) {
     const cudaStream_t s = (cudaStream_t)stream;

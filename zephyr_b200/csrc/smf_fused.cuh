@@ -89,6 +89,18 @@ __device__ __forceinline__ bool bad_fs(const FS<R> &z, R pmin) {
     return !ok;
 }
 
+// is_bad of a reconstructed FP64 state (models.cpp:58-63): r and p finite, r
+// positive, p not below the EoS's minimum; e = O(p / r) is then finite unless
+// r is below p by the whole exponent range.
+__device__ __forceinline__ bool bad_rp(double r, double p, double pmin) {
+    return !(r > fabs(p) * 0x1p-997 && p >= pmin && fabs(r + p) < INFINITY);
+}
+template <typename R>
+__device__ __forceinline__ bool bad_value(const FS<R> &z, R pmin) {
+    if constexpr (sizeof(R) == 8) return bad_rp(z.r, z.p, pmin);
+    else return bad_fs(z, pmin);
+}
+
 // phys flux along x of z (models.cpp:131-137 with the normal (1, 0))
 // (k = |v|^2)
 template <typename R>
@@ -142,6 +154,36 @@ __device__ __forceinline__ C4<R> hllc_fs(const FS<R> &L, const FS<R> &Rs, const 
     f.mu = rfma(SX, rfma(rs, SC, -ru), rfma(ru, X.u, X.p));
     f.mv = rfma(ru, X.v, rmul(SX, rfma(rs, X.v, -rmul(X.r, X.v))));
     f.E = rfma(radd(rE, X.p), X.u, rmul(SX, rfma(rs, Es, -rE)));
+    return f;
+}
+
+// The FP64 form of hllc_fs, in the marching kernel and in the tiles alike: the
+// supersonic cases as a choice of the upwind side instead of early returns.
+// VOTE: all lanes of the warp call it, and a warp without a subsonic face
+// leaves the star state out.
+template <bool VOTE>
+__device__ __forceinline__ C4<double> hllc_d(const FS<double> &L, const FS<double> &Rs, const EosR<double> &eos) {
+    const double cL = sound_ri(L, eos), cR = sound_ri(Rs, eos);
+    const double SL = smin_t(rsub(L.u, cL), rsub(Rs.u, cR)), SR = smax_t(radd(L.u, cL), radd(Rs.u, cR));
+    const double aL = rmul(L.r, rsub(SL, L.u)), aR = rmul(Rs.r, rsub(SR, Rs.u));
+    const double SC = rmul(rfma(-aL, L.u, rfma(aR, Rs.u, rsub(L.p, Rs.p))), rcp_nr(rsub(aR, aL)));
+    const bool subsonic = SL < 0.0 && SR > 0.0;
+    const bool left = subsonic ? SC >= 0.0 : SL >= 0.0;
+    const double r = left ? L.r : Rs.r, u = left ? L.u : Rs.u, v = left ? L.v : Rs.v, p = left ? L.p : Rs.p;
+    const double e = left ? L.e : Rs.e;
+    const double ru = rmul(r, u), EX = rfma(0.5, sq2(u, v), e), rE = rmul(r, EX);
+    C4<double> f{ru, rfma(ru, u, p), rmul(ru, v), rmul(radd(rE, p), u)};
+    if (VOTE ? __any_sync(0xffffffffu, subsonic) : subsonic) {
+        const double SX = left ? SL : SR, aX = left ? aL : aR;
+        const double rs = rmul(aX, rcp_nr(rsub(SX, SC)));
+        const double Es = rfma(rsub(SC, u), rfma(p, rcp_nr(aX), SC), EX);
+        if (subsonic) {
+            f.r = rfma(SX, rsub(rs, r), f.r);
+            f.mu = rfma(SX, rfma(rs, SC, -ru), f.mu);
+            f.mv = rfma(SX, rfma(rs, v, -rmul(r, v)), f.mv);
+            f.E = rfma(SX, rfma(rs, Es, -rE), f.E);
+        }
+    }
     return f;
 }
 
@@ -201,24 +243,72 @@ __device__ __forceinline__ R slope(int kind, R dL, R dR, R inv2h, R invh) {
 // The energy and 1 / r are the caller's.
 template <typename R>
 __device__ __forceinline__ FS<R> reconstruct(const FS<R> &z, R g0, R g1, R g2, R g3, R off, bool low) {
-    return FS<R>{rfma(g0, off, z.r), low ? radd(z.u, rmul(g1, off)) : rfma(g1, off, z.u),
-                 low ? radd(z.v, rmul(g2, off)) : rfma(g2, off, z.v), rfma(g3, off, z.p), R(0), R(0)};
+    const bool two = sizeof(R) == 4 && low;
+    return FS<R>{rfma(g0, off, z.r), two ? radd(z.u, rmul(g1, off)) : rfma(g1, off, z.u),
+                 two ? radd(z.v, rmul(g2, off)) : rfma(g2, off, z.v), rfma(g3, off, z.p), R(0), R(0)};
 }
-// The same at the half step's faces.
-template <typename R>
-__device__ __forceinline__ FS<R> reconstruct_half(const FS<R> &z, const R g[4], R off) {
-    return FS<R>{radd(z.r, rmul(g[0], off)), rfma(g[1], off, z.u), rfma(g[2], off, z.v), radd(z.p, rmul(g[3], off)),
+// Physical flux along an axis (ax: x) of a cell's value at its own face, for the
+// half step (sm_fluid.cpp:176-253); the cell's own value where that is bad.
+// rarely(bad, fix): runs fix where bad.
+template <typename R, typename F>
+__device__ __forceinline__ C4<R> half_flux(const FS<R> &c, const R g[4], R off, bool ax, const EosR<R> &eos, R igm1,
+                                           F &&rarely) {
+    if constexpr (sizeof(R) == 8) {
+        // r e = (p + gamma P0) / (gamma - 1) + r e0: no reciprocal density
+        double r = rfma(g[0], off, c.r), u = rfma(g[1], off, c.u), v = rfma(g[2], off, c.v), p = rfma(g[3], off, c.p);
+        double re = rfma(rfma(eos.gamma, eos.P0, p), igm1, rmul(r, eos.e0));
+        rarely(bad_rp(r, p, eos.pmin), [&] {
+            r = c.r, u = c.u, v = c.v, p = c.p;
+            re = rmul(r, c.e);
+        });
+        const double n = ax ? u : v, rn = rmul(r, n), E = rfma(rmul(0.5, r), sq2(u, v), re);
+        return C4<R>{rn, ax ? rfma(rn, u, p) : rmul(rn, u), ax ? rmul(rn, v) : rfma(rn, v, p), rmul(radd(E, p), n)};
+    } else {
+        FS<R> zm{radd(c.r, rmul(g[0], off)), rfma(g[1], off, c.u), rfma(g[2], off, c.v), radd(c.p, rmul(g[3], off)),
                  R(0), R(0)};
+        zm.ri = rcp_r(zm.r);
+        zm.e = energy_ri(eos, zm.p, zm.ri, igm1, true);
+        rarely(bad_fs(zm, eos.pmin), [&] { zm = c; });
+        if (ax) return flux_x(zm);
+        // flux along y: swap the velocity components
+        const C4<R> t = flux_x(FS<R>{zm.r, zm.v, zm.u, zm.p, zm.e, zm.ri});
+        return C4<R>{t.r, t.mv, t.mu, t.E};
+    }
+}
+// F += f w, and q -= k F
+template <typename R>
+__device__ __forceinline__ void add_half(double F[4], const C4<R> &f, double w) {
+    F[0] = rfma((double)f.r, w, F[0]);
+    F[1] = rfma((double)f.mu, w, F[1]);
+    F[2] = rfma((double)f.mv, w, F[2]);
+    F[3] = rfma((double)f.E, w, F[3]);
+}
+__device__ __forceinline__ void subtract(C4<double> &q, double k, const double F[4]) {
+    q.r = rfma(-k, F[0], q.r);
+    q.mu = rfma(-k, F[1], q.mu);
+    q.mv = rfma(-k, F[2], q.mv);
+    q.E = rfma(-k, F[3], q.E);
 }
 
-// A cell's outward flux sum from its faces' fluxes (low x, high x, low y, high y).
+// A cell's outward flux sum from its faces' fluxes (low x, high x, low y, high
+// y): MIXED in the slots' order; FP64 with the high x face last, which the march
+// has last.
 __device__ __forceinline__ double flux_sum(double xl, double xh, double yl, double yh, double hx, double hy) {
     return rfma(yh, hx, rfma(-yl, hx, rfma(xh, hy, -rmul(xl, hy))));
+}
+__device__ __forceinline__ double three_fluxes(double xl, double yl, double yh, double hx, double hy) {
+    return rfma(yh, hx, rfma(-yl, hx, -rmul(xl, hy)));
 }
 
 // Conserved variables of an FP64 primitive state (models.cpp:20-25).
 __device__ __forceinline__ C4<double> cons_of(double r, double u, double v, double e) {
     return C4<double>{r, r * u, r * v, r * rfma(0.5, sq2(u, v), e)};
+}
+
+// The same less k F.
+__device__ __forceinline__ C4<double> cons_less(double r, double u, double v, double e, double k, const double F[4]) {
+    return C4<double>{rfma(-k, F[0], r), rfma(r, u, -rmul(k, F[1])), rfma(r, v, -rmul(k, F[2])),
+                      rfma(r, rfma(0.5, sq2(u, v), e), -rmul(k, F[3]))};
 }
 
 // Conserved state of cell ic at t^n.
@@ -242,22 +332,44 @@ __device__ __forceinline__ P5<double> prim_ri(const C4<double> &q, const EosD &e
     return z;
 }
 
+template <bool VL, bool VR, typename R>
+__device__ __forceinline__ C4<R> hllc_any(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
+    if constexpr (sizeof(R) == 8) return hllc_d<false>(L, Rs, eos);
+    else return hllc_fs<VL, VR>(L, Rs, eos);
+}
+
 // Flux across a boundary face (WALL / ZOE, sm_fluid.cpp:69-79) from the
 // reconstructed state zm of its only cell, whose slot s_own it is: the ghost
 // state reflects the normal velocity at a wall; the flux is returned in the
-// +x / +y direction (negated when the cell lies on the face's high side).
-// Out of line: boundary faces are few, and one copy of the Riemann solver
-// serves all of them.
-template <typename R>
+// +x / +y direction.  FP64: in that direction's frame, as the march has it.
+// MIXED: in the frame of the cell's outward normal.  Out of line: boundary
+// faces are few, and one copy of the Riemann solver serves all of them.
+template <bool FIRST, typename R>
 __device__ __noinline__ C4<R> boundary_flux(FS<R> zm, int s_own, int bc, bool use_hll, EosR<R> eos, bool own_a) {
     FS<R> zp = zm;
     if (bc == BC_WALL) {
         if (s_own < 2) zp.u = -zp.u;
         else zp.v = -zp.v;
     }
+    if constexpr (sizeof(R) == 8) {
+        if (!own_a) {
+            const FS<R> t = zm;
+            zm = zp;
+            zp = t;
+        }
+        const int s = s_own | 1;  // the high slot of the axis: the + direction
+        to_local(s, zm.u, zm.v);
+        to_local(s, zp.u, zp.v);
+        C4<R> lf;
+        if (!use_hll) lf = hllc_any<true, true>(zm, zp, eos);
+        else if (s == 1) lf = hll_fs<FIRST, false, false>(zm, zp, eos);
+        else lf = hll_fs<true, true, true>(zm, zp, eos);
+        to_global(s, lf.mu, lf.mv);
+        return lf;
+    }
     to_local(s_own, zm.u, zm.v);
     to_local(s_own, zp.u, zp.v);
-    C4<R> lf = use_hll ? hll_fs<true, true, false>(zm, zp, eos) : hllc_fs<true, true>(zm, zp, eos);
+    C4<R> lf = use_hll ? hll_fs<true, true, false>(zm, zp, eos) : hllc_any<true, true>(zm, zp, eos);
     to_global(s_own, lf.mu, lf.mv);
     if (!own_a) {
         lf.r = -lf.r;
@@ -475,31 +587,14 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                 for (int s = 0; s < 4; ++s) {
                     const bool ax = s < 2;
                     const R off = s == 0 ? -halfx : (s == 1 ? halfx : (s == 2 ? -halfy : halfy));
-                    const R *gg = ax ? gx : gy;
-                    FS<R> zm = reconstruct_half(zc5, gg, off);
-                    zm.ri = rcp_r(zm.r);
-                    zm.e = energy_ri(eos, zm.p, zm.ri, igm1, true);
-                    if (bad_fs(zm, eos.pmin)) zm = zc5;
-                    C4<R> lf;
-                    if (ax) {
-                        lf = flux_x(zm);
-                    } else {  // flux along y: swap the velocity components
-                        const FS<R> zt{zm.r, zm.v, zm.u, zm.p, zm.e, zm.ri};
-                        const C4<R> t = flux_x(zt);
-                        lf = C4<R>{t.r, t.mv, t.mu, t.E};
-                    }
-                    const double w = (s == 0 || s == 2) ? -(ax ? m.hy : m.hx) : (ax ? m.hy : m.hx);
-                    F[0] += (double)lf.r * w;
-                    F[1] += (double)lf.mu * w;
-                    F[2] += (double)lf.mv * w;
-                    F[3] += (double)lf.E * w;
+                    const C4<R> lf = half_flux(zc5, ax ? gx : gy, off, ax, eos, igm1, [](bool on, auto &&fix) {
+                        if (on) fix();
+                    });
+                    add_half(F, lf, (s == 0 || s == 2) ? -(ax ? m.hy : m.hx) : (ax ? m.hy : m.hx));
                 }
                 const double half = 0.5 * coef;
                 C4<double> q = q0;
-                q.r -= half * F[0];
-                q.mu -= half * F[1];
-                q.mv -= half * F[2];
-                q.E -= half * F[3];
+                subtract(q, half, F);
                 double ri;
                 const P5<double> hd = prim_ri(q, a.eos, ri);
                 if (!bad64(hd, a.eos)) hz = down<R>(hd);
@@ -541,7 +636,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
                               !hi && !boundary);
         o.ri = rcp_r(o.r);
         o.e = energy_ri(eos, o.p, o.ri, igm1);
-        if (bad_fs(o, eos.pmin)) {
+        if (bad_value(o, eos.pmin)) {
             o = z;
             o.ri = rcp_r(z.r);
         }
@@ -570,7 +665,8 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
             zp.v = -t;
         }
         constexpr bool VR = DIR == 1, VL = VR || MODE == FUSED_HEUN_A;
-        C4<R> lf = (robust || a.flux == FLUX_HLL) ? hll_fs<VL, VR, DIR == 1>(zm, zp, eos) : hllc_fs<VL, VR>(zm, zp, eos);
+        C4<R> lf = (robust || a.flux == FLUX_HLL) ? hll_fs<VL, VR, DIR == 1>(zm, zp, eos)
+                                                  : hllc_any<VL, VR>(zm, zp, eos);
         if (DIR == 1) {
             const R t = lf.mu;
             lf.mu = -lf.mv;
@@ -584,7 +680,7 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
         const int s_own = own_a ? (dir == 0 ? 1 : 3) : (dir == 0 ? 0 : 2);
         const bool robust = PC && wt[gr][gc];
         const FS<R> zm = robust ? sc_ri(gr, gc) : recon(gr, gc, dir, own_a, true);
-        return boundary_flux(zm, s_own, m.bc[s_own], robust || a.flux == FLUX_HLL, eos, own_a);
+        return boundary_flux<MODE == FUSED_HEUN_A>(zm, s_own, m.bc[s_own], robust || a.flux == FLUX_HLL, eos, own_a);
     };
     // (predictor-corrector: the fluxes overwrite Z, which no thread reads
     // after phase 1)
@@ -620,26 +716,21 @@ __device__ __forceinline__ void step_tile(const SmfArgs &a, const Fields<R> &f, 
         double F[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            F[k] = flux_sum(FX[k][r - 1][l], FX[k][r][l], FY[k][r - 1][l - 1], FY[k][r - 1][l], hx, hy);
+            F[k] = MIXED ? flux_sum(FX[k][r - 1][l], FX[k][r][l], FY[k][r - 1][l - 1], FY[k][r - 1][l], hx, hy)
+                         : rfma(FX[k][r][l], hy,
+                                three_fluxes(FX[k][r - 1][l], FY[k][r - 1][l - 1], FY[k][r - 1][l], hx, hy));
         C4<double> q;
-        if (PC) {
-            q = C4<double>{Q[0][r][l], Q[1][r][l], Q[2][r][l], Q[3][r][l]};
-        } else if (MODE == FUSED_HEUN_B) {
-            // Q(z*) of the stage value
-            q = cons_of(Z[0][r + 1][l + 1], Z[1][r + 1][l + 1], Z[2][r + 1][l + 1], Z[4][r + 1][l + 1]);
-        } else {
-            q = q_n<R, MIXED>(f, ic);
-        }
-        q.r -= coef * F[0];
-        q.mu -= coef * F[1];
-        q.mv -= coef * F[2];
-        q.E -= coef * F[3];
         if (MODE == FUSED_HEUN_B) {
+            // Q(z*) of the stage value, its step, and the mean with Q(z^n)
+            q = cons_less(Z[0][r + 1][l + 1], Z[1][r + 1][l + 1], Z[2][r + 1][l + 1], Z[4][r + 1][l + 1], coef, F);
             const C4<double> q0 = q_n<R, MIXED>(f, ic);
             q.r = 0.5 * (q0.r + q.r);
             q.mu = 0.5 * (q0.mu + q.mu);
             q.mv = 0.5 * (q0.mv + q.mv);
             q.E = 0.5 * (q0.E + q.E);
+        } else {
+            q = PC ? C4<double>{Q[0][r][l], Q[1][r][l], Q[2][r][l], Q[3][r][l]} : q_n<R, MIXED>(f, ic);
+            subtract(q, coef, F);
         }
         double ri;
         zn = prim_ri(q, a.eos, ri);

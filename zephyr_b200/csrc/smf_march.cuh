@@ -53,26 +53,16 @@ __device__ __forceinline__ void rare(bool on, F &&fix) {
     }
 }
 
-// is_bad of a reconstructed FP64 state (models.cpp:58-63): r and p finite, r
-// positive, p not below the EoS's minimum; e = O(p / r) is then finite unless
-// r is below p by the whole exponent range.
-__device__ __forceinline__ bool bad_rp(double r, double p, double pmin) {
-    return !(r > fabs(p) * 0x1p-997 && p >= pmin && fabs(r + p) < INFINITY);
-}
-
 // A cell's value at the face centre `off` along an axis (FaceExtra::Direct,
 // face_extra.h:121-184) with slopes gr; the cell's own state where that is
 // bad.  All lanes of the warp call it.
 template <typename R>
 __device__ __forceinline__ FS<R> face_value(const FS<R> &h, const R gr[4], R off, bool low, const EosR<R> &eos,
                                             R igm1) {
-    FS<R> o = reconstruct(h, gr[0], gr[1], gr[2], gr[3], off, sizeof(R) == 4 && low);
+    FS<R> o = reconstruct(h, gr[0], gr[1], gr[2], gr[3], off, low);
     o.ri = rcp_r(o.r);
     o.e = energy_ri(eos, o.p, o.ri, igm1);
-    bool b;
-    if constexpr (sizeof(R) == 8) b = bad_rp(o.r, o.p, eos.pmin);
-    else b = bad_fs(o, eos.pmin);
-    rare(b, [&] {
+    rare(bad_value(o, eos.pmin), [&] {
         o = h;
         o.ri = rcp_r(h.r);
     });
@@ -91,46 +81,12 @@ __device__ __forceinline__ FS<R> half_step(const FS<R> &c, const C4<double> &q0,
     for (int s = 0; s < 4; ++s) {
         const bool ax = s < 2;
         const R off = s == 0 ? -k.halfx : (s == 1 ? k.halfx : (s == 2 ? -k.halfy : k.halfy));
-        const R *gg = ax ? gx : gy;
-        const double w = (s == 0 || s == 2) ? -(ax ? hy : hx) : (ax ? hy : hx);
-        C4<R> lf;
-        if constexpr (sizeof(R) == 8) {
-            // r e = (p + gamma P0) / (gamma - 1) + r e0: no reciprocal density
-            double r = c.r + gg[0] * off, u = c.u + gg[1] * off, v = c.v + gg[2] * off, p = c.p + gg[3] * off;
-            double re = (p + eos.gamma * eos.P0) * k.igm1 + r * eos.e0;
-            rare(bad_rp(r, p, eos.pmin), [&] {
-                r = c.r, u = c.u, v = c.v, p = c.p;
-                re = r * c.e;
-            });
-            const double n = ax ? u : v, rn = r * n;
-            lf.r = rn;
-            lf.mu = ax ? rn * u + p : rn * u;
-            lf.mv = ax ? rn * v : rn * v + p;
-            lf.E = (re + 0.5 * r * (u * u + v * v) + p) * n;
-        } else {
-            FS<R> zm = reconstruct_half(c, gg, off);
-            zm.ri = rcp_r(zm.r);
-            zm.e = energy_ri(eos, zm.p, zm.ri, k.igm1, true);
-            rare(bad_fs(zm, eos.pmin), [&] { zm = c; });
-            if (ax) {
-                lf = flux_x(zm);
-            } else {  // flux along y: swap the velocity components
-                const FS<R> zt{zm.r, zm.v, zm.u, zm.p, zm.e, zm.ri};
-                const C4<R> t = flux_x(zt);
-                lf = C4<R>{t.r, t.mv, t.mu, t.E};
-            }
-        }
-        F[0] += (double)lf.r * w;
-        F[1] += (double)lf.mu * w;
-        F[2] += (double)lf.mv * w;
-        F[3] += (double)lf.E * w;
+        const C4<R> lf = half_flux(c, ax ? gx : gy, off, ax, eos, k.igm1, [](bool on, auto &&fix) { rare(on, fix); });
+        add_half(F, lf, (s == 0 || s == 2) ? -(ax ? hy : hx) : (ax ? hy : hx));
     }
     const double half = 0.5 * coef;
     C4<double> q = q0;
-    q.r -= half * F[0];
-    q.mu -= half * F[1];
-    q.mv -= half * F[2];
-    q.E -= half * F[3];
+    subtract(q, half, F);
     double ri;
     const P5<double> hd = prim_ri(q, eosd, ri);
     const P5<R> hr = down<R>(hd);
@@ -139,40 +95,12 @@ __device__ __forceinline__ FS<R> half_step(const FS<R> &c, const C4<double> &q0,
     return h;
 }
 
-// HLLC in the frame (u normal, v tangential): hllc_fs with the supersonic
-// cases as a choice of the upwind side instead of early returns (FP64; the
-// FP32 form keeps hllc_fs).  All lanes of the warp call it.
-__device__ __forceinline__ C4<double> hllc_march(const FS<double> &L, const FS<double> &Rs, const EosR<double> &eos) {
-    const double cL = sqrt(eos.gamma * (L.p + eos.P0) * L.ri), cR = sqrt(eos.gamma * (Rs.p + eos.P0) * Rs.ri);
-    const double SL = smin_t(L.u - cL, Rs.u - cR);
-    const double SR = smax_t(L.u + cL, Rs.u + cR);
-    const double aL = L.r * (SL - L.u), aR = Rs.r * (SR - Rs.u);
-    const double SC = (L.p - Rs.p + aR * Rs.u - aL * L.u) * rcp_nr(aR - aL);
-    const bool subsonic = SL < 0.0 && SR > 0.0;
-    const bool left = subsonic ? SC >= 0.0 : SL >= 0.0;
-    const double r = left ? L.r : Rs.r, u = left ? L.u : Rs.u, v = left ? L.v : Rs.v, p = left ? L.p : Rs.p;
-    const double e = left ? L.e : Rs.e;
-    const double ru = r * u, EX = e + 0.5 * (u * u + v * v), rE = r * EX;
-    C4<double> f{ru, ru * u + p, ru * v, (rE + p) * u};
-    if (__any_sync(0xffffffffu, subsonic)) {
-        const double SX = left ? SL : SR, aX = left ? aL : aR;
-        const double rs = aX * rcp_nr(SX - SC);
-        const double Es = EX + (SC - u) * (SC + p * rcp_nr(aX));
-        if (subsonic) {
-            f.r += SX * (rs - r);
-            f.mu += SX * (rs * SC - ru);
-            f.mv += SX * (rs * v - r * v);
-            f.E += SX * (rs * Es - rE);
-        }
-    }
-    return f;
-}
 // VL, VR, Y: as hll_fs
 template <bool HLL, bool VL, bool VR, bool Y, typename R>
 __device__ __forceinline__ C4<R> march_flux(const FS<R> &L, const FS<R> &Rs, const EosR<R> &eos) {
     if constexpr (HLL) return hll_fs<VL, VR, Y>(L, Rs, eos);
     else if constexpr (sizeof(R) == 4) return hllc_fs<VL, VR>(L, Rs, eos);
-    else return hllc_march(L, Rs, eos);
+    else return hllc_d<true>(L, Rs, eos);
 }
 
 // The next step's CFL minimum (sm_fluid.cpp:104-111) over a warp's cells, with
@@ -342,8 +270,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
 
     FS<R> up{};     // row g - 1's state at its high face
     // row g - 1: the fluxes through its other three faces.  FP64: their sum.
-    // MIXED: the FP32 fluxes themselves (low x, low y, high y), summed in the
-    // tile's order, so that both forms give the same bits
+    // MIXED: the FP32 fluxes themselves (low x, low y, high y), whose sum takes
+    // them in another order (flux_sum)
     double acc[4];
     C4<R> fxl{}, fyl{}, fyh{};
     int sm = 0, sc = 1, sp = 2, sn = 3;  // state slots of rows g - 1, g, g + 1, g + 2
@@ -449,27 +377,28 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
         // ---- update of row g - 1 -------------------------------------------
         if (g > i_lo) {
             if (MODE != FUSED_HEUN_A && (g - i_lo) % 16 == 1) cfl.refresh(f.slot_nxt);
-            // Heun's second stage starts from the stage value's own Q
-            C4<double> q = MODE == FUSED_HEUN_B
-                               ? cons_of(ring.z[sm][0][l], ring.z[sm][1][l], ring.z[sm][2][l], ring.z[sm][4][l])
-                               : base(sm, bm);
+            double F[4];
             if constexpr (MIXED) {
-                q.r -= coef * flux_sum(fxl.r, fx.r, fyl.r, fyh.r, hx, hy);
-                q.mu -= coef * flux_sum(fxl.mu, fx.mu, fyl.mu, fyh.mu, hx, hy);
-                q.mv -= coef * flux_sum(fxl.mv, fx.mv, fyl.mv, fyh.mv, hx, hy);
-                q.E -= coef * flux_sum(fxl.E, fx.E, fyl.E, fyh.E, hx, hy);
+                F[0] = flux_sum(fxl.r, fx.r, fyl.r, fyh.r, hx, hy);
+                F[1] = flux_sum(fxl.mu, fx.mu, fyl.mu, fyh.mu, hx, hy);
+                F[2] = flux_sum(fxl.mv, fx.mv, fyl.mv, fyh.mv, hx, hy);
+                F[3] = flux_sum(fxl.E, fx.E, fyl.E, fyh.E, hx, hy);
             } else {
-                q.r -= coef * (acc[0] + (double)fx.r * hy);
-                q.mu -= coef * (acc[1] + (double)fx.mu * hy);
-                q.mv -= coef * (acc[2] + (double)fx.mv * hy);
-                q.E -= coef * (acc[3] + (double)fx.E * hy);
+                F[0] = rfma(fx.r, hy, acc[0]);
+                F[1] = rfma(fx.mu, hy, acc[1]);
+                F[2] = rfma(fx.mv, hy, acc[2]);
+                F[3] = rfma(fx.E, hy, acc[3]);
             }
-            if (MODE == FUSED_HEUN_B) {
-                const C4<double> qn = base(sm, bm);
-                q.r = 0.5 * (qn.r + q.r);
-                q.mu = 0.5 * (qn.mu + q.mu);
-                q.mv = 0.5 * (qn.mv + q.mv);
-                q.E = 0.5 * (qn.E + q.E);
+            C4<double> q = base(sm, bm);
+            if (MODE == FUSED_HEUN_B) {  // starts from the stage value's own Q
+                const C4<double> t = cons_less(ring.z[sm][0][l], ring.z[sm][1][l], ring.z[sm][2][l], ring.z[sm][4][l],
+                                               coef, F);
+                q.r = 0.5 * (q.r + t.r);
+                q.mu = 0.5 * (q.mu + t.mu);
+                q.mv = 0.5 * (q.mv + t.mv);
+                q.E = 0.5 * (q.E + t.E);
+            } else {
+                subtract(q, coef, F);
             }
             store_cell<R, MIXED, MODE>(a, f, g - 1, j, live, q, wm, cfl);
         }
@@ -479,10 +408,10 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
         if constexpr (MIXED) {
             fxl = fx, fyl = fb, fyh = fy;
         } else {
-            acc[0] = (-(double)fx.r * hy - (double)fb.r * hx) + (double)fy.r * hx;
-            acc[1] = (-(double)fx.mu * hy - (double)fb.mu * hx) + (double)fy.mu * hx;
-            acc[2] = (-(double)fx.mv * hy - (double)fb.mv * hx) + (double)fy.mv * hx;
-            acc[3] = (-(double)fx.E * hy - (double)fb.E * hx) + (double)fy.E * hx;
+            acc[0] = three_fluxes(fx.r, fb.r, fy.r, hx, hy);
+            acc[1] = three_fluxes(fx.mu, fb.mu, fy.mu, hx, hy);
+            acc[2] = three_fluxes(fx.mv, fb.mv, fy.mv, hx, hy);
+            acc[3] = three_fluxes(fx.E, fb.E, fy.E, hx, hy);
         }
         up = face_value<R>(h, gx, k.halfx, false, eos, k.igm1);
         if (iso && (wc | wp) != 0) up = own;

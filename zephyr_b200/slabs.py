@@ -26,7 +26,9 @@ contiguous in memory):
 
 A rank's result equals the single-domain step's on its owned rows: bit for
 bit when the local rectangles reproduce the global mesh's coordinates (a
-dyadic cell size), to rounding otherwise.
+dyadic cell size), to rounding otherwise.  (A slab's steps may run another
+kernel than the whole mesh's would, which are chosen by size: the kernels of a
+family give the same bits.)
 
 The communicator is pluggable: `TorchComm` uses torch.distributed (NCCL on
 GPU buffers, gloo on host buffers; one process per GPU), `LocalComm` runs
