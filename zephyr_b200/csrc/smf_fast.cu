@@ -96,22 +96,19 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
 // The form by size, measured on B200 (us per step, march / tile):
 //   predictor-corrector  2048^2 314 / 332, 1200^2 111 / 122, 1024^2 85 / 89, 896^2 71 / 66
 //   Heun                 2048^2 430 / 479, 1200^2 162 / 175, 1024^2 125 / 134, 896^2 104 / 101
-// so the march from 16 rows per segment on (1024^2).  Below, the tile kernel;
-// where its grid would leave a quarter of the SMs without a block, tiles of 2
-// rows instead of 14 (64^2 10.7 -> 8.7 us, 200^2 11.3 -> 10.9, 256^2 15 -> 17).
-// All forms give the same bits, so that the slabs of a mesh may each take the
-// form of their own size.
+// so the march from 16 rows per segment on (1024^2).  Below, the tile kernel,
+// with 4-row tiles on small meshes (small_tiles).  All forms give the same bits,
+// so that the slabs of a mesh may each take the form of their own size.
 constexpr int MARCH_MIN_ROWS_PC = 16, MARCH_MIN_ROWS_HEUN = 16;
 void launch_step(const SmfArgs &a, const Fields<double> &f, int mode, void *stream) {
     const cudaStream_t s = (cudaStream_t)stream;
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_FAST_MARCH_MINB);
     constexpr int TH = ZG_FAST_FUSED_TH;
-    const long long tiles = (long long)((a.mesh.ny + 29) / 30) * ((a.mesh.nx + TH - 1) / TH);
     if (tiled::march_limiter(a.limiter) &&
         sp.rows >= (mode == tiled::FUSED_PC ? MARCH_MIN_ROWS_PC : MARCH_MIN_ROWS_HEUN))
         tiled::march_dispatch<double, false, ZG_FAST_MARCH_MINB>(a, f, mode, sp, s);
-    else if (4 * tiles <= 3 * 148)
-        tiled::fused_dispatch<double, false, 2, 4>(a, f, mode, s);
+    else if (tiled::small_tiles(a.mesh, mode == tiled::FUSED_PC ? 3 : 4))
+        tiled::fused_dispatch<double, false, tiled::SMALL_TH, tiled::SMALL_MINB>(a, f, mode, s);
     else
         tiled::fused_dispatch<double, false, TH, ZG_FAST_FUSED_MINB>(a, f, mode, s);
 }

@@ -808,6 +808,23 @@ __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<
     step_tile<R, MIXED, MODE, LIM, TH, false>(a, f, k);
 }
 
+// Meshes that leave the 14-row tiles few blocks run tiles of 4 rows, as long as
+// their blocks are resident at once (192 threads each; FP64's predictor-corrector
+// has registers for three on an SM, the others for four): one block's phases,
+// one after the other, are what a step of such a mesh takes.  us a step, 4 rows /
+// 14 rows (van Albada HLLC): FP64 predictor-corrector 64^2 7.3 / 9.0, 129x67 8.8 /
+// 9.1, 200^2 8.8 / 10.3, 220x210 8.7 / 10.3; Heun 200^2 15.8 / 18.4; MIXED Heun
+// 129x67 11.0 / 12.1, 240^2 14.8 / 15.5 (2 rows: 200^2 8.5 and 14.8, but 2 waves
+// from 210^2 on; MIXED Heun with MC 129x67 16.7 against 12.5).
+// One wave of 14-row tiles on more than half of the SMs is launched normally:
+// blocks of the next kernel that wait beside it cost more than the launch saves
+// (240^2 12.4 us with the dependent launch, 10.3 without; 256^2, more than one
+// wave, 12.5 with, 14.4 without).
+constexpr int SMALL_TH = 4, SMALL_MINB = 3, SMS = 148;
+inline bool small_tiles(const StructMesh &m, int resident) {
+    return (long long)((m.ny + 29) / 30) * ((m.nx + SMALL_TH - 1) / SMALL_TH) <= (long long)resident * SMS;
+}
+
 // Launch one stage of the fused step on `stream` (dynamic shared memory of
 // FusedLayout::bytes, above the 48 KB default).
 template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
@@ -823,7 +840,11 @@ inline void launch_fused_stage(const SmfArgs &a, const Fields<R> &f, cudaStream_
     }
     dim3 block(32, TH + 2);
     dim3 grid((a.mesh.ny + 29) / 30, (a.mesh.nx + TH - 1) / TH);
-    launch_after(kern, grid, block, L::bytes, s, a, f, step_const<R>(a));
+    const long long blocks = (long long)grid.x * grid.y;
+    if (TH == SMALL_TH || 2 * blocks <= SMS || blocks > SMS)
+        launch_after(kern, grid, block, L::bytes, s, a, f, step_const<R>(a));
+    else
+        kern<<<grid, block, L::bytes, s>>>(a, f, step_const<R>(a));
 }
 
 // One stage (FUSED_PC, FUSED_HEUN_A or FUSED_HEUN_B) with the limiter

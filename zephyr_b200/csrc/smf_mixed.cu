@@ -106,18 +106,17 @@ void launch_to_prim(int n, const Fields<float> &f, EosD eos, PrimPtr z, void *st
 //   predictor-corrector  2048^2 250 / 257, 1700^2 177 / 181, 1448^2 135 / 135, 1024^2 76 / 72
 //   Heun                 2048^2 321 / 387, 1200^2 126 / 142, 896^2 78 / 81, 768^2 66 / 63
 // (the predictor's FP64 half makes the march's registers the limit).  Small
-// meshes take tiles of 2 rows instead of 14, as in the FP64 form.
+// meshes take tiles of 4 rows instead of 14, as in the FP64 form.
 constexpr int MARCH_MIN_ROWS_PC = 32, MARCH_MIN_ROWS_HEUN = 10;
 void launch_step(const SmfArgs &a, const Fields<float> &f, int mode, void *stream) {
     const cudaStream_t s = (cudaStream_t)stream;
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_MIXED_MARCH_MINB);
     constexpr int TH = ZG_MIXED_FUSED_TH;
-    const long long tiles = (long long)((a.mesh.ny + 29) / 30) * ((a.mesh.nx + TH - 1) / TH);
     if (tiled::march_limiter(a.limiter) && a.mesh.xper && a.mesh.yper &&
         sp.rows >= (mode == tiled::FUSED_PC ? MARCH_MIN_ROWS_PC : MARCH_MIN_ROWS_HEUN))
         tiled::march_dispatch<float, true, ZG_MIXED_MARCH_MINB>(a, f, mode, sp, s);
-    else if (4 * tiles <= 3 * 148)
-        tiled::fused_dispatch<float, true, 2, 4>(a, f, mode, s);
+    else if (tiled::small_tiles(a.mesh, 4))
+        tiled::fused_dispatch<float, true, tiled::SMALL_TH, tiled::SMALL_MINB>(a, f, mode, s);
     else
         tiled::fused_dispatch<float, true, TH, ZG_MIXED_FUSED_MINB>(a, f, mode, s);
 }
