@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(BLOCK, ZG_ADJ_VF_MINB) k_vjp_faces(Grid g, CF4
                 hllc_vjp<double>(L, R, gamma, ml, Lb, Rb, gpart);
             } else {
                 S gb = S(0);
-                hllc_vjp<S>(L, R, S(gamma), ml, Lb, Rb, gb);
+                hllc_vjp_symmetric<S>(L, R, S(gamma), ml, Lb, Rb, gb);
                 gpart += (double)gb;
             }
             S *fb = yface ? fby : fbx;
