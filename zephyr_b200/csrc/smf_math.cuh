@@ -49,11 +49,11 @@ __host__ __device__ inline T smax_t(T a, T b) { return (a < b) ? b : a; }
 // a / b where a is often exactly zero (velocities of a gas at rest, fractions of
 // an absent material, a contact's pressure jump): CUDA's division takes a call
 // out of line for the whole warp when a lane's numerator is zero or its result
-// is not a normal number.  The zero is taken around the division; the result
-// is a / b up to the sign of a zero (NaN for b = 0 or NaN).
+// is not a normal number.  The zero is taken around the division, with its
+// sign; the result is a / b.
 __host__ __device__ inline double div_z(double a, double b) {
     const bool z = a == 0.0;
-    const double q = (z ? 0x1p-100 : a) / b;
+    const double q = (z ? copysign(0x1p-100, a) : a) / b;
     return z ? q * 0.0 : q;
 }
 // both non-zero and of one sign (false with a NaN)
