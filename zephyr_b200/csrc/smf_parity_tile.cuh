@@ -119,7 +119,8 @@ template <class Put>
 __device__ __forceinline__ bool hllc_both(const FState &A, const FState &B, const EosD &eos, Put &&put) {
     const double cA = eos.sound_speed_rP(A.r, A.p), cB = eos.sound_speed_rP(B.r, B.p);
     const double SL = smin(A.n - cA, B.n - cB), SR = smax(A.n + cA, B.n + cB);
-    if (!((SR - SL) + (fabs(A.t) + fabs(B.t)) < CUDART_INF)) return false;
+    // (both sides' own values: the minimum of a number and a NaN is the first)
+    if (!(fabs(cA + cB + A.n + B.n) + (fabs(A.t) + fabs(B.t)) < CUDART_INF)) return false;
     if (SL >= 0.0 || SR <= 0.0) {  // each cell tests its own side first
         const F4 fA = flux_n(A.r, A.n, A.t, A.p, A.e), fB = flux_n(B.r, B.n, B.t, B.p, B.e);
         put(0, SL >= 0.0 ? fA : fB);
