@@ -59,7 +59,7 @@ struct StructMesh {
     const double *cx, *cy;    // cell centres (SqQuad vs<0,0>)
     const double *fxm, *fym;  // mid-edge coordinates 0.5*(X[i]+X[i+1]), 0.5*(Y[j]+Y[j+1])
     const double *inc2x, *inc2y;  // squared incircle extents per column / row
-    double inc2min;               // their smallest value
+    double inc2min;               // the cells' smallest; 0: they differ by more than 1e-4
     double hx, hy, vol;
 };
 

@@ -1119,7 +1119,13 @@ int zg_mesh_rectangle(zg_ctx *c, int nx, int ny, double x_min, double x_max, dou
     m.fym = c->d_geo + ofy;
     m.inc2x = c->d_geo + oix;
     m.inc2y = c->d_geo + oiy;
-    m.inc2min = std::min(*std::min_element(i2x.begin(), i2x.end()), *std::min_element(i2y.begin(), i2y.end()));
+    {
+        const auto x = std::minmax_element(i2x.begin(), i2x.end()), y = std::minmax_element(i2y.begin(), i2y.end());
+        const double lo = std::min(*x.first, *y.first), hi = std::min(*x.second, *y.second);
+        // cells that differ in size by their coordinates' rounding (far from the
+        // origin, 1e12 cells away): no common bound, every CFL term is formed
+        m.inc2min = hi <= lo * 1.0001 ? lo : 0.0;
+    }
     c->box[0] = x_min;
     c->box[1] = x_max;
     c->box[2] = y_min;
