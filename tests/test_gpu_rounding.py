@@ -4,7 +4,7 @@ neither on its place in the mesh (interior or border tile) nor on the kernel
 that the mesh's size picks.
 
 * Periodic data moved by any number of cells: the result moved, bit for bit.
-* MIXED on a small mesh (tiles of 2 rows), on a middle one (14 rows) and on a
+* MIXED on a small mesh (tiles of 4 rows), on a middle one (14 rows) and on a
   large one (the march) made of copies of the small one: the same bits.
 * MIXED results stay the ones they were: digests of states that the one tile
   kernel of 14 rows gave when it ran every mesh.
@@ -97,7 +97,7 @@ def test_mixed_forms_give_the_same_bits(gpu_lib, scheme, flux, wait):
         w = np.zeros((n, n), np.int32)
         w.ravel()[[5, 700, 701, 4095]] = (1, 2, 3, 3)
     small, ds = advance(gpu_lib, z, "MIXED", scheme, flux, "van Albada", 4, wait=w)
-    for kx, ky in ((8, 7), (31, 29)):
+    for kx, ky in ((8, 7), (34, 32)):
         big, db = advance(gpu_lib, [np.tile(q, (kx, ky)) for q in z], "MIXED", scheme, flux, "van Albada", 4,
                           box=(float(kx), float(ky)), wait=None if w is None else np.tile(w, (kx, ky)))
         assert db == ds

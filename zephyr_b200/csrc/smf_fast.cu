@@ -93,13 +93,14 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
 #ifndef ZG_FAST_MARCH_MINB
 #define ZG_FAST_MARCH_MINB 4
 #endif
-// The form by size, measured on B200 (us per step, march / tile):
-//   predictor-corrector  2048^2 314 / 332, 1200^2 111 / 122, 1024^2 85 / 89, 896^2 71 / 66
-//   Heun                 2048^2 430 / 479, 1200^2 162 / 175, 1024^2 125 / 134, 896^2 104 / 101
-// so the march from 16 rows per segment on (1024^2).  Below, the tile kernel,
-// with 4-row tiles on small meshes (small_tiles).  All forms give the same bits,
-// so that the slabs of a mesh may each take the form of their own size.
-constexpr int MARCH_MIN_ROWS_PC = 16, MARCH_MIN_ROWS_HEUN = 16;
+// The form by size, measured on B200 (us per step of van Albada HLLC, march / tile):
+//   predictor-corrector  1024^2 88 / 84, 1700^2 226 / 222, 2048^2 315 / 318, 3072^2 657 / 704, 6000x1200 514 / 539
+//   Heun                 1024^2 124 / 125, 1700^2 312 / 322, 2048^2 430 / 464, 3072^2 908 / 1017
+// so the march from 48 and 16 rows per segment on (2048^2: 64, 1700^2: 45, 1024^2:
+// 16; HLL gains 3 % more).  Below, the tile kernel, with 4-row tiles on small
+// meshes (small_tiles).  All forms give the same bits, so that the slabs of a
+// mesh may each take the form of their own size.
+constexpr int MARCH_MIN_ROWS_PC = 48, MARCH_MIN_ROWS_HEUN = 16;
 void launch_step(const SmfArgs &a, const Fields<double> &f, int mode, void *stream) {
     const cudaStream_t s = (cudaStream_t)stream;
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_FAST_MARCH_MINB);

@@ -798,7 +798,7 @@ template <typename R, bool MIXED, int MODE, int LIM, int TH, int MINB>
 __global__ void __launch_bounds__(32 * (TH + 2), MINB) k_step(SmfArgs a, Fields<R> f, StepConst<R> k) {
     after_previous();
     const int i0 = blockIdx.y * TH, j0 = blockIdx.x * 30;
-    // (a limiter chosen at run time: one copy of its code, see march_limiter)
+    // (a limiter chosen at run time: one copy of its code)
     if constexpr (LIM >= 0) {
         if (i0 >= 2 && i0 + TH + 2 <= a.mesh.nx && j0 >= 2 && j0 + 32 <= a.mesh.ny) {
             step_tile<R, MIXED, MODE, LIM, TH, true>(a, f, k);

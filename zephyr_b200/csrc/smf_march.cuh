@@ -21,12 +21,14 @@
 // they look: an atomic minimum per cell on the one CFL slot (190 us at 1024^2
 // against 88 with one per warp), and bad-value fallbacks as selects instead of
 // branches under a warp vote (5 % of a step at 2048^2).
-// Measured (B200, one step, FP64 / MIXED): 2048^2 predictor-corrector 353 ->
-// 310 / 293 -> 247 us, Heun 542 -> 430 / 457 -> 305 us.
-// MIXED gives the tile's bits: the same FP32 formulas with their roundings
-// written out (smf_tiled.cuh), the same order of the flux sum.  That holds on
-// periodic axes; a boundary face is another instance in the tile (seen from its
-// own cell), so MIXED marches only on rectangles that are periodic both ways.
+// Measured (B200, one step of van Albada HLLC, march / tile with the same
+// formulas): FP64 predictor-corrector 2048^2 315 / 318 us, 3072^2 657 / 704, Heun
+// 2048^2 430 / 464; MIXED 246 / 248, 514 / 544, 304 / 375 (before the march: FP64
+// 353 and 542, MIXED 293 and 457 at 2048^2).
+// Both forms give the same bits: shared formulas with written-out roundings.  In
+// MIXED that holds on periodic axes (a boundary face is another instance in the
+// tile, seen from its own cell), so MIXED marches only on rectangles that are
+// periodic both ways.
 #pragma once
 
 #include "smf_fused.cuh"
@@ -200,7 +202,7 @@ struct MarchRing {
     double b[BASE ? 3 : 1][BASE ? 4 : 1][BASE ? 32 : 1];
 };
 
-template <typename R, bool MIXED, int MODE, int LIM, bool HLL, int MINB>
+template <typename R, bool MIXED, int MODE, bool HLL, int MINB>
 __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_constant__ SmfArgs a,
                                                                   const __grid_constant__ Fields<R> f,
                                                                   const __grid_constant__ StepConst<R> k, int strips,
@@ -317,8 +319,8 @@ __global__ void __launch_bounds__(32 * MARCH_WARPS, MINB) k_march(const __grid_c
                 if (jlow) nB = q == 2 && m.bc[2] == BC_WALL ? -c : c;
                 if (jhigh) nT = q == 2 && m.bc[3] == BC_WALL ? -c : c;
             }
-            gx[q] = slope<LIM, R>(a.limiter, nL - c, nR - c, k.inv2hx, k.invhx);
-            gy[q] = slope<LIM, R>(a.limiter, nB - c, nT - c, k.inv2hy, k.invhy);
+            gx[q] = slope<LIM_VANALBADA1, R>(LIM_VANALBADA1, nL - c, nR - c, k.inv2hx, k.invhx);
+            gy[q] = slope<LIM_VANALBADA1, R>(LIM_VANALBADA1, nB - c, nT - c, k.inv2hy, k.invhy);
         }
         // ---- state the faces are reconstructed from: the half step, or z --
         if (PC) {
@@ -449,27 +451,28 @@ inline MarchSplit march_split(const StructMesh &m, int minb) {
     }
     return MarchSplit{(int)strips, rows};
 }
-template <typename R, bool MIXED, int MODE, int LIM, int MINB>
+template <typename R, bool MIXED, int MODE, int MINB>
 inline void launch_march(const SmfArgs &a, const Fields<R> &f, const MarchSplit &sp, cudaStream_t s) {
     const int segs = (a.mesh.nx + sp.rows - 1) / sp.rows;
     const unsigned blocks = (unsigned)(((long long)segs * sp.strips + MARCH_WARPS - 1) / MARCH_WARPS);
     const dim3 nt(32 * MARCH_WARPS);
     if (a.flux == FLUX_HLL)
-        k_march<R, MIXED, MODE, LIM, true, MINB><<<blocks, nt, 0, s>>>(a, f, step_const<R>(a), sp.strips, sp.rows);
+        k_march<R, MIXED, MODE, true, MINB><<<blocks, nt, 0, s>>>(a, f, step_const<R>(a), sp.strips, sp.rows);
     else
-        k_march<R, MIXED, MODE, LIM, false, MINB><<<blocks, nt, 0, s>>>(a, f, step_const<R>(a), sp.strips, sp.rows);
+        k_march<R, MIXED, MODE, false, MINB><<<blocks, nt, 0, s>>>(a, f, step_const<R>(a), sp.strips, sp.rows);
 }
 // The march runs van Albada 1, whose slope has a closed form.  The limiters that
 // are formed from the general refit keep more values alive, and 128 registers a
 // thread leave too few warps to cover their divisions: tile against march, FP64
-// at 2000^2 on smooth data: MC 402 / 461, minmod 365 / 395, van Leer 368 / 399 us
-// (van Albada 1: 338 / 314 at 2048^2); MIXED at 2048^2 MC 291 / 318.
+// predictor-corrector at 2000^2 on smooth data, with the formulas both had at
+// first: MC 402 / 461, minmod 365 / 395, van Leer 368 / 399 us (van Albada 1 338 /
+// 314 at 2048^2); MIXED at 2048^2 MC 291 / 318.
 inline bool march_limiter(int lim) { return lim == LIM_VANALBADA1; }
 template <typename R, bool MIXED, int MINB>
 inline void march_dispatch(const SmfArgs &a, const Fields<R> &f, int mode, const MarchSplit &sp, cudaStream_t s) {
-    if (mode == FUSED_PC) launch_march<R, MIXED, FUSED_PC, LIM_VANALBADA1, MINB>(a, f, sp, s);
-    else if (mode == FUSED_HEUN_A) launch_march<R, MIXED, FUSED_HEUN_A, LIM_VANALBADA1, MINB>(a, f, sp, s);
-    else launch_march<R, MIXED, FUSED_HEUN_B, LIM_VANALBADA1, MINB>(a, f, sp, s);
+    if (mode == FUSED_PC) launch_march<R, MIXED, FUSED_PC, MINB>(a, f, sp, s);
+    else if (mode == FUSED_HEUN_A) launch_march<R, MIXED, FUSED_HEUN_A, MINB>(a, f, sp, s);
+    else launch_march<R, MIXED, FUSED_HEUN_B, MINB>(a, f, sp, s);
 }
 
 }  // namespace tiled

@@ -102,12 +102,12 @@ void launch_to_prim(int n, const Fields<float> &f, EosD eos, PrimPtr z, void *st
 #ifndef ZG_MIXED_MARCH_MINB
 #define ZG_MIXED_MARCH_MINB 5
 #endif
-// The form by size, measured on B200 (us per step, march / tile):
-//   predictor-corrector  2048^2 250 / 257, 1700^2 177 / 181, 1448^2 135 / 135, 1024^2 76 / 72
-//   Heun                 2048^2 321 / 387, 1200^2 126 / 142, 896^2 78 / 81, 768^2 66 / 63
+// The form by size, measured on B200 (us per step of van Albada HLLC, march / tile):
+//   predictor-corrector  1700^2 177 / 173, 2048^2 246 / 248, 3072^2 514 / 544, 4096^2 889 / 960, 6000x1200 426 / 417
+//   Heun                 896^2 74 / 73, 1024^2 92 / 98, 2048^2 304 / 375, 3072^2 631 / 824
 // (the predictor's FP64 half makes the march's registers the limit).  Small
 // meshes take tiles of 4 rows instead of 14, as in the FP64 form.
-constexpr int MARCH_MIN_ROWS_PC = 32, MARCH_MIN_ROWS_HEUN = 10;
+constexpr int MARCH_MIN_ROWS_PC = 48, MARCH_MIN_ROWS_HEUN = 11;
 void launch_step(const SmfArgs &a, const Fields<float> &f, int mode, void *stream) {
     const cudaStream_t s = (cudaStream_t)stream;
     const tiled::MarchSplit sp = tiled::march_split(a.mesh, ZG_MIXED_MARCH_MINB);
