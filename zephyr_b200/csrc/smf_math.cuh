@@ -53,8 +53,8 @@ __host__ __device__ inline T smax_t(T a, T b) { return (a < b) ? b : a; }
 // sign; the result is a / b.
 __host__ __device__ inline double div_z(double a, double b) {
     const bool z = a == 0.0;
-    const double q = (z ? copysign(0x1p-100, a) : a) / b;
-    return z ? q * 0.0 : q;
+    const double q = (z ? 0x1p-100 : a) / b;
+    return z ? a * q : q;
 }
 // both non-zero and of one sign (false with a NaN)
 template <typename T>
