@@ -94,8 +94,8 @@ void launch_faces(const SmfArgs &a, const Fields<double> &f, int mode, void *str
 #define ZG_FAST_MARCH_MINB 4
 #endif
 // The form by size, measured on B200 (us per step of van Albada HLLC, march / tile):
-//   predictor-corrector  1024^2 88 / 84, 1700^2 226 / 222, 2048^2 315 / 318, 3072^2 657 / 704, 6000x1200 514 / 539
-//   Heun                 1024^2 124 / 125, 1700^2 312 / 322, 2048^2 430 / 464, 3072^2 908 / 1017
+//   predictor-corrector  1024^2 86 / 83, 1700^2 223 / 222, 2048^2 310 / 317, 3072^2 648 / 704, 6000x1200 506 / 539
+//   Heun                 1024^2 124 / 125, 1700^2 312 / 322, 2048^2 430 / 463, 3072^2 909 / 1016
 // so the march from 48 and 16 rows per segment on (2048^2: 64, 1700^2: 45, 1024^2:
 // 16; HLL gains 3 % more).  Below, the tile kernel, with 4-row tiles on small
 // meshes (small_tiles).  All forms give the same bits, so that the slabs of a

@@ -22,8 +22,8 @@
 // against 88 with one per warp), and bad-value fallbacks as selects instead of
 // branches under a warp vote (5 % of a step at 2048^2).
 // Measured (B200, one step of van Albada HLLC, march / tile with the same
-// formulas): FP64 predictor-corrector 2048^2 315 / 318 us, 3072^2 657 / 704, Heun
-// 2048^2 430 / 464; MIXED 246 / 248, 514 / 544, 304 / 375 (before the march: FP64
+// formulas): FP64 predictor-corrector 2048^2 310 / 317 us, 3072^2 648 / 704, Heun
+// 2048^2 430 / 463; MIXED 246 / 248, 514 / 544, 304 / 375 (before the march: FP64
 // 353 and 542, MIXED 293 and 457 at 2048^2).
 // Both forms give the same bits: shared formulas with written-out roundings.  In
 // MIXED that holds on periodic axes (a boundary face is another instance in the
